@@ -395,8 +395,18 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, const Traver
 // Persistent warps refill a lane with the next ray of the queue when fewer
 // than st.refillBelow of its 32 rays are still traversing (incoherent
 // secondary rays end at very different times); tuned per scene, 10 by default
-// (what the autotuner picks on the benchmark heightfield, 8 to 10).
+// (of 4 to 28, within 0.4 % of the best on heightfields, closed rooms and
+// instances: 95.4 ms per 1080p, 64 spp heightfield render against 97.8 at 4,
+// 99.6 at 16 and 104.1 at 24).
+// A ray that ends waits for the refill in its lane: its result is then handled
+// with those of the warp's other ended rays (about 20) instead of at once, where
+// nearly every step stopped the whole warp at the round trip of a queue append or
+// a radiance update made by one or two lanes. Heightfield render (1080p, 64 spp)
+// 95.5 -> 89.8 ms, a frame under a sky (960 x 540, 4 spp) 1.67 -> 1.26 ms.
 constexpr uint32_t kRefillBelow = 10;
+
+// Largest block of the persistent traversal kernels (LaunchShape::traversalThreads).
+constexpr uint32_t kTraversalThreadsMax = 128;
 
 // Closest hit of the bounce's extend queue. Rays that hit are appended (one
 // warp ballot and one atomic per step) to the hit queue with their full path
@@ -453,16 +463,57 @@ __global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f
     TraversalCounts cnt{0, 0};
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
-    float4 O4 = make_float4(0.f, 0.f, 0.f, 0.f), D4 = O4, T4 = O4;
+    // What the traversal does not need of a lane's ray: its throughput and the ids in O.w
+    // and D.w wait here (this thread's words only) instead of in registers.
+    __shared__ float4 rayT[kTraversalThreadsMax];
+    __shared__ float2 rayIds[kTraversalThreadsMax];
     const uint32_t sc = (PRIMARY || BATCH) ? *f.sampleCount : 0u;
-    bool alive = false, more = true;
+    bool alive = false, ended = false, more = true;
     while (true) {
-        const uint32_t idle = __ballot_sync(kFull, !alive && more);
+        // The rays that ended since the last refill, all lanes at once: one append to the
+        // hit queue, its atomic in flight beside the refill's.
+        const bool hit = ended && base(t).hitSlot != 0xffffffffu;
+        const uint32_t hits = __ballot_sync(kFull, hit);
+        const uint32_t idle = more ? __ballot_sync(kFull, !alive) : 0u;
+        const uint32_t hitLeader = hits ? __ffs(hits) - 1u : 0u;
+        const uint32_t leader = idle ? __ffs(idle) - 1u : 0u;
+        uint32_t slot = 0, first = 0;
+        if (hits && lane == hitLeader)
+            slot = atomicAdd(hitCounter, __popc(hits));
+        if (idle && lane == leader)
+            first = atomicAdd(work, __popc(idle));
+        if (ended) {
+            if (!base(t).ok)
+                atomicOr(f.errorFlag, 1u);
+            if (!hit) {
+                const float2 ids = rayIds[threadIdx.x];
+                if (s.sky.enabled) {
+                    sky_miss<BATCH>(s, f, st, bounce, f4(ray_origin(t), ids.x), f4(ray_direction(t), ids.y),
+                                    rayT[threadIdx.x], aov);
+                } else if (aov) {
+                    // a primary miss sees the disabled sky: black guide values (PathTracing.h:48-52)
+                    const uint32_t pathIx = path_ix(__float_as_uint(ids.x));
+                    if (pathIx < wh) {
+                        f.albedo[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        f.normals[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                }
+            }
+        }
+        if (hits) {
+            slot = __shfl_sync(kFull, slot, hitLeader) + __popc(hits & ((1u << lane) - 1u));
+            if (hit) {
+                const uint32_t prim = __float_as_uint(__ldg(s.bvhTris + 3u * base(t).hitSlot).w);
+                const float2 ids = rayIds[threadIdx.x];
+                __stcs(hq + slot, f4(ray_origin(t), ids.x));
+                __stcs(hq + slot + cap, f4(ray_direction(t), ids.y));
+                __stcs(hq + slot + 2 * cap, rayT[threadIdx.x]);
+                __stcs(f.hits + slot, make_uint4(encode_bary(base(t).u, base(t).v), hit_instance(t), prim,
+                                                 __float_as_uint(base(t).tmax)));
+            }
+        }
+        ended = false;
         if (idle) {
-            const uint32_t leader = __ffs(idle) - 1u;
-            uint32_t first = 0;
-            if (lane == leader)
-                first = atomicAdd(work, __popc(idle));
             first = __shfl_sync(kFull, first, leader);
             // batched: the item of the first new sample of this refill, found by the
             // whole warp (the first sample ids of 32 items per load and a ballot, in
@@ -480,66 +531,45 @@ __global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f
                         break;  // items are in sample order: none later starts at or before it
                 }
             }
-            if (!alive && more) {
-                const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
-                if (i < count) {
-                    if (BATCH ? i >= carried : PRIMARY) {
-                        float3 O, D;
-                        float T;
-                        uint32_t item = warpItem;
-                        const uint32_t pathIx = BATCH ? freshBase + (i - carried) : camera_order(f, i);
-                        primary_ray<false, BATCH>(f, cam, st, pathIx, sc, O, D, T, &item);
-                        // a batch path keeps its sample id in O.w and item | bounce | flags in D.w
-                        O4 = f4(O, u2f(BATCH ? pathIx : pack_path(pathIx, 0)));
-                        D4 = f4(D, BATCH ? u2f(batch_pack(0u, 0u, item)) : 0.f);
-                        T4 = make_float4(T, T, T, 1.f);
-                        f.radiance[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    } else {
-                        O4 = __ldcs(in + i);
-                        D4 = __ldcs(in + i + cap);
-                        T4 = __ldcs(in + i + 2 * cap);
-                    }
-                    traversal_begin(t, f3(O4), f3(D4), st.rayEpsilon, kDstMax,
-                                    BATCH ? item_root(f, batch_item_of(__float_as_uint(D4.w))) : 0u);
-                    alive = true;
+            const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
+            if (!alive && i < count) {
+                float4 O4, D4, T4;
+                if (BATCH ? i >= carried : PRIMARY) {
+                    float3 O, D;
+                    float T;
+                    uint32_t item = warpItem;
+                    const uint32_t pathIx = BATCH ? freshBase + (i - carried) : camera_order(f, i);
+                    primary_ray<false, BATCH>(f, cam, st, pathIx, sc, O, D, T, &item);
+                    // a batch path keeps its sample id in O.w and item | bounce | flags in D.w
+                    O4 = f4(O, u2f(BATCH ? pathIx : pack_path(pathIx, 0)));
+                    D4 = f4(D, BATCH ? u2f(batch_pack(0u, 0u, item)) : 0.f);
+                    T4 = make_float4(T, T, T, 1.f);
+                    f.radiance[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
                 } else {
-                    more = false;
+                    O4 = __ldcs(in + i);
+                    D4 = __ldcs(in + i + cap);
+                    T4 = __ldcs(in + i + 2 * cap);
                 }
+                rayT[threadIdx.x] = T4;
+                rayIds[threadIdx.x] = make_float2(O4.w, D4.w);
+                traversal_begin(t, f3(O4), f3(D4), st.rayEpsilon, kDstMax,
+                                BATCH ? item_root(f, batch_item_of(__float_as_uint(D4.w))) : 0u);
+                alive = true;
             }
+            more = first + __popc(idle) < count;
         }
         if (!__any_sync(kFull, alive))
             break;
+        // with the queue empty there is nothing to refill: the warp's rays run out together
+        const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
-            bool done = false;
-            if (alive)
-                done = traversal_step<false, COUNT, LAYOUT>(t, stack, s, &cnt);
-            const bool hit = done && base(t).hitSlot != 0xffffffffu;
-            const uint32_t slot = warp_append(hitCounter, hit);
-            if (done) {
-                if (!base(t).ok)
-                    atomicOr(f.errorFlag, 1u);
-                if (hit) {
-                    const uint32_t prim = __float_as_uint(__ldg(s.bvhTris + 3u * base(t).hitSlot).w);
-                    __stcs(hq + slot, O4);
-                    __stcs(hq + slot + cap, D4);
-                    __stcs(hq + slot + 2 * cap, T4);
-                    __stcs(f.hits + slot, make_uint4(encode_bary(base(t).u, base(t).v), hit_instance(t), prim,
-                                                     __float_as_uint(base(t).tmax)));
-                } else if (s.sky.enabled) {
-                    sky_miss<BATCH>(s, f, st, bounce, O4, D4, T4, aov);
-                } else if (aov) {
-                    // a primary miss sees the disabled sky: black guide values (PathTracing.h:48-52)
-                    const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
-                    if (pathIx < wh) {
-                        f.albedo[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                        f.normals[pathIx] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    }
-                }
+            if (alive && traversal_step<false, COUNT, LAYOUT>(t, stack, s, &cnt)) {
                 alive = false;
+                ended = true;
             }
             active = __ballot_sync(kFull, alive);
-        } while (uint32_t(__popc(active)) >= st.refillBelow);
+        } while (uint32_t(__popc(active)) >= below);
     }
     if (COUNT)
         add_counts(f.traversal, cnt);
@@ -1151,51 +1181,55 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
     uint32_t visibleCnt = 0;
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
-    uint32_t ray = 0, pathIx = 0;
-    bool alive = false, more = true;
+    __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
+    bool alive = false, ended = false, more = true;
     while (true) {
-        const uint32_t idle = __ballot_sync(kFull, !alive && more);
-        if (idle) {
-            const uint32_t leader = __ffs(idle) - 1u;
-            uint32_t base = 0;
-            if (lane == leader)
-                base = atomicAdd(work, __popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (!alive && more) {
-                const uint32_t i = base + __popc(idle & ((1u << lane) - 1u));
-                if (i < count) {
-                    const float4 O4 = __ldcs(f.shadow + i);
-                    const float4 L4 = __ldcs(f.shadow + i + cap);
-                    ray = i;
-                    pathIx = __float_as_uint(O4.w);
-                    const uint32_t root =
-                        BATCH ? __float_as_uint(__ldcs(reinterpret_cast<const float*>(f.shadow + i + 2 * cap) + 3))
-                              : 0u;
-                    traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon), root);
-                    alive = true;
-                } else {
-                    more = false;
-                }
+        // The rays that ended since the last refill, all lanes at once: the contribution of
+        // the unoccluded ones, while the refill's atomic is in flight.
+        const uint32_t idle = more ? __ballot_sync(kFull, !alive) : 0u;
+        const uint32_t leader = idle ? __ffs(idle) - 1u : 0u;
+        uint32_t first = 0;
+        if (idle && lane == leader)
+            first = atomicAdd(work, __popc(idle));
+        if (ended) {
+            if (!base(t).ok)
+                atomicOr(f.errorFlag, 1u);
+            if (base(t).hitSlot == 0xffffffffu) {
+                const uint2 ids = rayIds[threadIdx.x];
+                const float4 T4 = __ldcs(f.shadow + ids.x + 2 * cap);
+                const float4 r = f.radiance[ids.y];
+                f.radiance[ids.y] = make_float4(r.x + T4.x, r.y + T4.y, r.z + T4.z, r.w);
+                if (COUNT)
+                    ++visibleCnt;
             }
+            ended = false;
+        }
+        if (idle) {
+            first = __shfl_sync(kFull, first, leader);
+            const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
+            if (!alive && i < count) {
+                const float4 O4 = __ldcs(f.shadow + i);
+                const float4 L4 = __ldcs(f.shadow + i + cap);
+                rayIds[threadIdx.x] = make_uint2(i, __float_as_uint(O4.w));
+                const uint32_t root =
+                    BATCH ? __float_as_uint(__ldcs(reinterpret_cast<const float*>(f.shadow + i + 2 * cap) + 3)) : 0u;
+                traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon), root);
+                alive = true;
+            }
+            more = first + __popc(idle) < count;
         }
         if (!__any_sync(kFull, alive))
             break;
+        // with the queue empty there is nothing to refill: the warp's rays run out together
+        const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
             if (alive && traversal_step<true, COUNT, LAYOUT>(t, stack, s, &cnt)) {
-                if (!base(t).ok)
-                    atomicOr(f.errorFlag, 1u);
-                if (base(t).hitSlot == 0xffffffffu) {
-                    const float4 T4 = __ldcs(f.shadow + ray + 2 * cap);
-                    float4 r = f.radiance[pathIx];
-                    f.radiance[pathIx] = make_float4(r.x + T4.x, r.y + T4.y, r.z + T4.z, r.w);
-                    if (COUNT)
-                        ++visibleCnt;
-                }
                 alive = false;
+                ended = true;
             }
             active = __ballot_sync(kFull, alive);
-        } while (uint32_t(__popc(active)) >= st.refillBelow);
+        } while (uint32_t(__popc(active)) >= below);
     }
     if (COUNT) {
         add_counts(f.traversal + 2, cnt);
@@ -1830,51 +1864,56 @@ __global__ void __launch_bounds__(128) adjoint_connect_kernel(SceneView s, Frame
     const uint32_t lane = lane_id();
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
-    uint32_t ray = 0, pathIx = 0;
-    bool alive = false, more = true;
+    __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
+    bool alive = false, ended = false, more = true;
     while (true) {
-        const uint32_t idle = __ballot_sync(kFull, !alive && more);
-        if (idle) {
-            const uint32_t leader = __ffs(idle) - 1u;
-            uint32_t base = 0;
-            if (lane == leader)
-                base = atomicAdd(work, __popc(idle));
-            base = __shfl_sync(kFull, base, leader);
-            if (!alive && more) {
-                const uint32_t i = base + __popc(idle & ((1u << lane) - 1u));
-                if (i < count) {
-                    const float4 O4 = __ldcs(f.shadow + i);
-                    const float4 L4 = __ldcs(f.shadow + i + cap);
-                    ray = i;
-                    pathIx = __float_as_uint(O4.w);
-                    traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon));
-                    alive = true;
-                } else {
-                    more = false;
-                }
+        // the rays that ended since the last refill, all lanes at once (as connect_kernel)
+        const bool visible = ended && base(t).hitSlot == 0xffffffffu;
+        const uint32_t vis = __ballot_sync(kFull, visible);
+        const uint32_t idle = more ? __ballot_sync(kFull, !alive) : 0u;
+        const uint32_t visLeader = vis ? __ffs(vis) - 1u : 0u;
+        const uint32_t leader = idle ? __ffs(idle) - 1u : 0u;
+        uint32_t slot = 0, first = 0;
+        if (vis && lane == visLeader)
+            slot = atomicAdd(visCounter, __popc(vis));
+        if (idle && lane == leader)
+            first = atomicAdd(work, __popc(idle));
+        if (ended && !base(t).ok)
+            atomicOr(f.errorFlag, 1u);
+        if (vis) {
+            slot = __shfl_sync(kFull, slot, visLeader) + __popc(vis & ((1u << lane) - 1u));
+            if (visible) {
+                const uint2 ids = rayIds[threadIdx.x];
+                const float4 T4 = __ldcs(f.shadow + ids.x + 2 * cap);
+                const float4 r = a.lrem[ids.y];
+                a.lrem[ids.y] = make_float4(r.x - T4.x, r.y - T4.y, r.z - T4.z, r.w);
+                a.visible[slot] = ids.x;
             }
+        }
+        ended = false;
+        if (idle) {
+            first = __shfl_sync(kFull, first, leader);
+            const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
+            if (!alive && i < count) {
+                const float4 O4 = __ldcs(f.shadow + i);
+                const float4 L4 = __ldcs(f.shadow + i + cap);
+                rayIds[threadIdx.x] = make_uint2(i, __float_as_uint(O4.w));
+                traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon));
+                alive = true;
+            }
+            more = first + __popc(idle) < count;
         }
         if (!__any_sync(kFull, alive))
             break;
+        const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
-            bool visible = false;
             if (alive && traversal_step<true, false>(t, stack, s, nullptr)) {
-                if (!base(t).ok)
-                    atomicOr(f.errorFlag, 1u);
-                if (base(t).hitSlot == 0xffffffffu) {
-                    const float4 T4 = __ldcs(f.shadow + ray + 2 * cap);
-                    const float4 r = a.lrem[pathIx];
-                    a.lrem[pathIx] = make_float4(r.x - T4.x, r.y - T4.y, r.z - T4.z, r.w);
-                    visible = true;
-                }
                 alive = false;
+                ended = true;
             }
-            const uint32_t slot = warp_append(visCounter, visible);
-            if (visible)
-                a.visible[slot] = ray;
             active = __ballot_sync(kFull, alive);
-        } while (uint32_t(__popc(active)) >= st.refillBelow);
+        } while (uint32_t(__popc(active)) >= below);
     }
 }
 

@@ -716,6 +716,10 @@ struct TravOf<true> {
 // The result fields of either traversal.
 TR_HD const Traversal& base(const Traversal& t) { return t; }
 TR_HD const Traversal& base(const TraversalTL& r) { return r.t; }
+TR_HD float3 ray_origin(const Traversal& t) { return t.O; }
+TR_HD float3 ray_origin(const TraversalTL& r) { return r.wO; }
+TR_HD float3 ray_direction(const Traversal& t) { return t.D; }
+TR_HD float3 ray_direction(const TraversalTL& r) { return r.wD; }
 TR_HD uint32_t hit_instance(const Traversal&) { return 0u; }
 TR_HD uint32_t hit_instance(const TraversalTL& r) { return r.hitInst; }
 
