@@ -37,6 +37,13 @@ SceneAccel build_accel(const tr_scene_desc& desc, const std::vector<uint32_t>& m
     for (uint32_t i = 0; i < desc.instance_count; ++i) {
         const uint32_t mi = desc.instances[i].mesh;
         out.instInfo.push_back(make_uint2(out.meshRoot[mi], meshTriBase[mi]));
+        float inv[12];
+        inverse_3x4(desc.instances[i].transform, inv);
+        for (int r = 0; r < 3; ++r) {
+            const float* row = inv + 4 * r;
+            if (!(std::fabs(row[0]) + std::fabs(row[1]) + std::fabs(row[2]) < kQuantMaxDirection))
+                out.quantizable = false;
+        }
         const Aabb& b = meshBox[mi];
         if (!(b.lo[0] <= b.hi[0]))
             continue;  // empty mesh
@@ -75,6 +82,12 @@ SceneAccel build_accel(const tr_scene_desc& desc, const std::vector<uint32_t>& m
     for (uint32_t p : wideTop.triPrim)
         out.tlasInst.push_back(ids[p]);
     return out;
+}
+
+bool quantize_accel(const SceneAccel& acc, bool wanted, std::vector<QuantNode>& nodes,
+                    std::vector<QuantNode>& tlasNodes)
+{
+    return wanted && acc.quantizable && quantize_nodes(acc.nodes, nodes) && quantize_nodes(acc.tlasNodes, tlasNodes);
 }
 
 } // namespace tr

@@ -19,6 +19,7 @@ struct SceneAccel {
     std::vector<WideNode> tlasNodes;  // two-level scenes: BVH over the instances' world boxes
     std::vector<uint32_t> tlasInst;    // instance of each leaf slot of tlasNodes
     std::vector<uint2> instInfo;       // per instance: (BVH root node, first triangle of its mesh)
+    bool quantizable = true;           // no instance magnifies directions past kQuantMaxDirection
 };
 
 // meshTriBase: first triangle of each mesh in the concatenated shading
@@ -26,5 +27,10 @@ struct SceneAccel {
 // node 0, no instance level.
 SceneAccel build_accel(const tr_scene_desc& desc, const std::vector<uint32_t>& meshTriBase,
                        const BvhBuildOptions& opt);
+
+// The scene's nodes with quantized child boxes, where the node mode asks for them
+// (quantized_nodes) and the scene allows them; false: the fp32 nodes serve.
+bool quantize_accel(const SceneAccel& acc, bool wanted, std::vector<QuantNode>& nodes,
+                    std::vector<QuantNode>& tlasNodes);
 
 } // namespace tr

@@ -250,9 +250,10 @@ tr_status upload_texture(Context* c, const tr_texture_desc& t)
 // scene view at them.
 tr_status upload_bvh(Context* c, const SceneAccel& acc)
 {
-    const bool quant = quantized_nodes(acc.nodes.size() + acc.tlasNodes.size(), c->nodeMode, !acc.tlasNodes.empty());
-    const std::vector<QuantNode> qnodes = quant ? quantize_nodes(acc.nodes) : std::vector<QuantNode>{};
-    const std::vector<QuantNode> qtlas = quant ? quantize_nodes(acc.tlasNodes) : std::vector<QuantNode>{};
+    std::vector<QuantNode> qnodes, qtlas;
+    const bool quant = quantize_accel(
+        acc, quantized_nodes(acc.nodes.size() + acc.tlasNodes.size(), c->nodeMode, !acc.tlasNodes.empty()), qnodes,
+        qtlas);
     const void* nodeSrc = quant ? static_cast<const void*>(qnodes.data()) : static_cast<const void*>(acc.nodes.data());
     const void* tlasSrc = quant ? static_cast<const void*>(qtlas.data()) : static_cast<const void*>(acc.tlasNodes.data());
     const size_t nodeSize = quant ? sizeof(QuantNode) : sizeof(WideNode);

@@ -409,9 +409,9 @@ tr_status tr_batch_create(const tr_config* config, const tr_batch_item* items, u
         off = align256(off + std::max<size_t>(bytes, 16));
         return o;
     };
-    // the node layout of the concatenated BVHs (fp32 child boxes while they fit L2)
-    const bool quant = quantized_nodes(nodes.size(), 0u);
-    const std::vector<QuantNode> qnodes = quant ? quantize_nodes(nodes) : std::vector<QuantNode>{};
+    // the node layout of the concatenated BVHs (one-level scenes: by their node count)
+    std::vector<QuantNode> qnodes;
+    const bool quant = quantized_nodes(nodes.size(), 0u) && quantize_nodes(nodes, qnodes);
     const void* nodeSrc = quant ? static_cast<const void*>(qnodes.data()) : static_cast<const void*>(nodes.data());
     const size_t nodeBytes = nodes.size() * (quant ? sizeof(QuantNode) : sizeof(WideNode));
     const size_t oNodes = take(nodeBytes);

@@ -617,9 +617,9 @@ Cwbvh collapse_to_cwbvh(const BinaryBvh& bvh, const float* positions, const uint
         t.join();
     return out;
 }
-std::vector<QuantNode> quantize_nodes(const std::vector<WideNode>& nodes)
+bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& out)
 {
-    std::vector<QuantNode> out(nodes.size());
+    out.assign(nodes.size(), QuantNode{});
     for (size_t n = 0; n < nodes.size(); ++n) {
         const WideNode& w = nodes[n];
         const uint32_t meta[2] = {w.hdr.z, w.hdr.w};
@@ -648,10 +648,12 @@ std::vector<QuantNode> quantize_nodes(const std::vector<WideNode>& nodes)
                 std::frexp(extent / 255.0, &ex);
                 e = ex;
             }
-            e = std::max(-126, std::min(e, 127));
+            if (!(extent < double(kQuantMaxExtent)))
+                return false;
+            e = std::max(-100, e);
             scale[a] = std::ldexp(1.0, e);
             w0[a] = f2u(box.lo[a]);
-            w0[3] |= uint32_t(e + 127) << (8 * a);
+            w0[3] |= uint32_t(e + kQuantStepExponent) << (8 * a);
         }
         uint32_t imask = 0;
         for (int sl = 0; sl < 8; ++sl) {
@@ -675,7 +677,7 @@ std::vector<QuantNode> quantize_nodes(const std::vector<WideNode>& nodes)
         o.w[3] = make_uint4(q[2][0], q[2][1], q[3][0], q[3][1]);
         o.w[4] = make_uint4(q[4][0], q[4][1], q[5][0], q[5][1]);
     }
-    return out;
+    return true;
 }
 
 } // namespace tr

@@ -63,18 +63,30 @@ Cwbvh collapse_to_cwbvh(const BinaryBvh& bvh, const float* positions, const uint
                         uint32_t sahMaxLeaf = 0);
 
 // The same nodes with 8-bit quantized child boxes (rounded outwards against
-// each node's box, the union of its children's).
-std::vector<QuantNode> quantize_nodes(const std::vector<WideNode>& nodes);
+// each node's box, the union of its children's). False (out undefined) when a
+// node's extent is kQuantMaxExtent or more (or not finite): its steps along a ray
+// of the smallest direction that the traversal tells from zero (1e-20) would not
+// fit a float at the traversal's scale (2^42 * step * 1e20 < 2^127).
+constexpr float kQuantMaxExtent = 0x1p24f;
+bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& out);
+// Largest magnification of a ray's direction into an instance's space that the
+// quantized layout takes (its reciprocal, at the traversal's scale, must not be
+// denormal); scenes beyond keep fp32 child boxes.
+constexpr float kQuantMaxDirection = 0x1p20f;
 
-// Node layout of an uploaded BVH: mode 0 (auto) keeps fp32 child boxes while the
-// nodes fit kWideNodeBudget (they then stay in L2 beside the wavefront
-// buffers) and the scene has one level (the two-level traversal holds more
-// state, and fp32 nodes make it spill), 1 always fp32, 2 always quantized.
-// Returns true for quantized.
-constexpr size_t kWideNodeBudget = size_t(64) << 20;
+// Node layout of an uploaded BVH: mode 0 (auto) keeps fp32 child boxes for one-level
+// scenes of up to kWideNodeMax nodes, 1 always fp32, 2 always quantized. Returns true
+// for quantized.
+// The fp32 test needs fewer instructions and 2.6 times the bytes through L1, whose data
+// pipe bounds it as soon as a warp's lanes visit different nodes. 720p frames, fp32 /
+// quantized: closed room (3 nodes) 2087 / 2178 us; heightfields of 142 nodes 1419 / 1434,
+// 519 nodes 1695 / 1688, 3305 nodes 2148 / 2079, 13351 nodes 2480 / 2354. The two are
+// within 3 % of each other up to the line; two-level scenes keep the quantized layout (a
+// small one would gain 7 % with fp32, whose larger traversal state spills).
+constexpr size_t kWideNodeMax = 4096;
 inline bool quantized_nodes(size_t nodeCount, uint32_t mode, bool twoLevel = false)
 {
-    return mode == 2u || (mode == 0u && (twoLevel || nodeCount * sizeof(WideNode) > kWideNodeBudget));
+    return mode == 2u || (mode == 0u && (twoLevel || nodeCount > kWideNodeMax));
 }
 
 } // namespace tr

@@ -89,8 +89,7 @@ struct AliasEntry {
 // WideNode, child boxes in fp32, 208 bytes:
 //   hdr: child_base, tri_base, meta[0..3], meta[4..7]
 //   lo[a][slot], hi[a][slot]: the child boxes per axis (empty slot: +inf / -inf)
-// No per-child byte unpacking in the traversal, whose issue slots bound it;
-// used while the nodes stay L2-resident (the heightfield's 214k nodes: 45 MB).
+// For small BVHs, whose nodes a warp's lanes share (see kWideNodeMax).
 struct alignas(16) WideNode {
     uint4 hdr;
     float lo[3][8];
@@ -104,8 +103,9 @@ static_assert(sizeof(WideNode) == 208, "WideNode must stay 208 bytes");
 //   w2: qlo.x[0..7], qlo.y[0..7]
 //   w3: qlo.z[0..7], qhi.x[0..7]
 //   w4: qhi.y[0..7], qhi.z[0..7]
-// e are biased exponents (scale = 2^(e-127)); a child box is p + q * scale,
-// rounded outwards. For BVHs too large for L2.
+// e are exponents plus kQuantStepExponent (scale = 2^(e - 142): the traversal takes
+// a step's distance times 2^142); a child box is p + q * scale, rounded outwards.
+constexpr int kQuantStepExponent = 142;
 struct alignas(16) QuantNode {
     uint4 w[5];
 };

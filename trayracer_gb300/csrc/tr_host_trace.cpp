@@ -28,10 +28,9 @@ extern "C" tr_status tr_trace_host(const tr_scene_desc* desc, const float* O4, c
     opt.threads = desc->build_threads;
     const FlatScene fs = flatten_scene(*desc);
     const SceneAccel acc = build_accel(*desc, fs.meshTriBase, opt);
-    const bool quant = (any_hit & 2) != 0;
+    std::vector<QuantNode> qnodes, qtlas;
+    const bool quant = quantize_accel(acc, (any_hit & 2) != 0, qnodes, qtlas);
     any_hit &= 1;
-    const std::vector<QuantNode> qnodes = quant ? quantize_nodes(acc.nodes) : std::vector<QuantNode>{};
-    const std::vector<QuantNode> qtlas = quant ? quantize_nodes(acc.tlasNodes) : std::vector<QuantNode>{};
     SceneView s{};
     s.nodes = quant ? static_cast<const void*>(qnodes.data()) : static_cast<const void*>(acc.nodes.data());
     s.quantNodes = quant ? 1u : 0u;

@@ -445,7 +445,7 @@ __device__ __noinline__ void sky_miss(const SceneView& s, const FrameView& f, co
 // new samples (their camera rays are made here), so the pool stays full.
 // Blocks of 64 or 128 threads (a launch parameter, LaunchShape::traversalThreads):
 // the kernel works per warp; 64 registers, 32 resident warps per SM.
-template <bool COUNT, bool BATCH, bool PRIMARY, bool TL, int LAYOUT = kLayoutScene>
+template <bool COUNT, bool BATCH, bool PRIMARY, bool TL, int LAYOUT>
 __global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
                                                      Camera cam)
 {
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f
                 }
                 rayT[threadIdx.x] = T4;
                 rayIds[threadIdx.x] = make_float2(O4.w, D4.w);
-                traversal_begin(t, f3(O4), f3(D4), st.rayEpsilon, kDstMax,
+                traversal_begin<LAYOUT>(t, f3(O4), f3(D4), kDstMax,
                                 BATCH ? item_root(f, batch_item_of(__float_as_uint(D4.w))) : 0u);
                 alive = true;
             }
@@ -564,7 +564,7 @@ __global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f
         const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
-            if (alive && traversal_step<false, COUNT, LAYOUT>(t, stack, s, &cnt)) {
+            if (alive && traversal_step<false, COUNT, LAYOUT>(t, st.rayEpsilon, stack, s, &cnt)) {
                 alive = false;
                 ended = true;
             }
@@ -1169,7 +1169,7 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(FrameView f, SortView
 // the latency of its node fetches; 31.3 against 33.1 ms of shadow rays per 1080p, 64 spp
 // heightfield step at 72 registers and 7 blocks). Two-level traversal holds more state and
 // keeps its own register count (it would spill 100-210 bytes at 56).
-template <bool COUNT, bool BATCH, bool TL, int LAYOUT = kLayoutScene>
+template <bool COUNT, bool BATCH, bool TL, int LAYOUT>
 __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, FrameView f, Settings st,
                                                                    uint32_t bounce)
 {
@@ -1213,7 +1213,7 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
                 rayIds[threadIdx.x] = make_uint2(i, __float_as_uint(O4.w));
                 const uint32_t root =
                     BATCH ? __float_as_uint(__ldcs(reinterpret_cast<const float*>(f.shadow + i + 2 * cap) + 3)) : 0u;
-                traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon), root);
+                traversal_begin<LAYOUT>(t, f3(O4), f3(L4), L4.w - (2 * st.rayEpsilon), root);
                 alive = true;
             }
             more = first + __popc(idle) < count;
@@ -1224,7 +1224,7 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
         const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
-            if (alive && traversal_step<true, COUNT, LAYOUT>(t, stack, s, &cnt)) {
+            if (alive && traversal_step<true, COUNT, LAYOUT>(t, st.rayEpsilon, stack, s, &cnt)) {
                 alive = false;
                 ended = true;
             }
@@ -1853,8 +1853,8 @@ __global__ void __launch_bounds__(kAdjointThreads, 4) adjoint_shade_kernel(Scene
 // Visibility of the replay's NEE rays (as connect_kernel): an unoccluded ray
 // takes its contribution off the path's remaining radiance and is listed for
 // nee_grad_kernel.
-template <bool TL>
-__global__ void __launch_bounds__(128) adjoint_connect_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
+template <bool TL, int LAYOUT>
+__global__ void __launch_bounds__(128, TL ? 1 : 9) adjoint_connect_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
                                                               AdjointView a)
 {
     const uint32_t count = __ldcg(f.counters + kShadowCounterBase + bounce);
@@ -1898,7 +1898,7 @@ __global__ void __launch_bounds__(128) adjoint_connect_kernel(SceneView s, Frame
                 const float4 O4 = __ldcs(f.shadow + i);
                 const float4 L4 = __ldcs(f.shadow + i + cap);
                 rayIds[threadIdx.x] = make_uint2(i, __float_as_uint(O4.w));
-                traversal_begin(t, f3(O4), f3(L4), st.rayEpsilon, L4.w - (2 * st.rayEpsilon));
+                traversal_begin<LAYOUT>(t, f3(O4), f3(L4), L4.w - (2 * st.rayEpsilon));
                 alive = true;
             }
             more = first + __popc(idle) < count;
@@ -1908,7 +1908,7 @@ __global__ void __launch_bounds__(128) adjoint_connect_kernel(SceneView s, Frame
         const uint32_t below = more ? st.refillBelow : 1u;
         uint32_t active;
         do {
-            if (alive && traversal_step<true, false>(t, stack, s, nullptr)) {
+            if (alive && traversal_step<true, false, LAYOUT>(t, st.rayEpsilon, stack, s, nullptr)) {
                 alive = false;
                 ended = true;
             }
@@ -2201,10 +2201,14 @@ cudaError_t launch_adjoint(const SceneView& s0, const FrameView& f, const Camera
             adjoint_shade_kernel<true><<<gradBlocks, kAdjointThreads, smem, stream>>>(s, f, fwd, bounce, a);
         else
             adjoint_shade_kernel<false><<<gradBlocks, kAdjointThreads, 0, stream>>>(s, f, fwd, bounce, a);
-        if (s.tlasNodes)
-            adjoint_connect_kernel<true><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
+        if (s.tlasNodes && !s.quantNodes)
+            adjoint_connect_kernel<true, kLayoutWide><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
+        else if (s.tlasNodes)
+            adjoint_connect_kernel<true, kLayoutQuant><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
+        else if (s.quantNodes)
+            adjoint_connect_kernel<false, kLayoutQuant><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
         else
-            adjoint_connect_kernel<false><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
+            adjoint_connect_kernel<false, kLayoutWide><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
         if (useSmem)
             nee_grad_kernel<true><<<gradBlocks, kAdjointThreads, smem, stream>>>(s, f, bounce, a);
         else

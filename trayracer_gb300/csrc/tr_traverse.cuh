@@ -5,7 +5,9 @@
 // traversal following Ylitie, Karras and Laine (HPG 2017): node groups on a
 // short stack, octant-ordered child slots, 8-bit quantized child boxes decoded
 // against the ray with one FMA per slab, leaf triangles visited as a bit mask.
-// Node words are fetched as 128-bit read-only loads.
+// Node words are fetched as 128-bit read-only loads (256-bit loads of nodes padded
+// to 224 or 256 bytes were 5 to 18 % slower: nodes at such strides meet in the same
+// L1 banks).
 //
 // OptiX semantics kept: no face culling (Tracer/Resources/Model.cpp:270),
 // closest hit over [tmin, tmax], any-hit termination for shadow rays
@@ -146,15 +148,33 @@ TR_HD bool intersect_triangle(const float3& O, const float3& D, const float4& a,
     return true;
 }
 
-// float(byte i of w), exact. On the device the byte is placed in the low
-// mantissa bits of 2^23 (one byte permute) and 2^23 subtracted (one add), which
-// avoids the quarter-rate integer-to-float conversion.
-TR_HD float byte_to_float(uint32_t w, int i)
+// The quantized layout's box test reads a child plane's byte q without a conversion: 128 q,
+// taken as float bits, is the denormal number q * 2^-142 (exact; denormal operands cost the
+// FMA nothing). Its factor, a quantization step's distance along the ray times 2^142, only
+// fits a float because the test's time runs 2^100 times slower (kQuantTime * t for t) - powers
+// of two throughout, so every distance rounds as at full scale. The ray's reciprocal direction
+// is kept at kQuantTime.
+constexpr float kQuantTime = 0x1p-100f;
+
+// byte i of w (on the device an integer dot product, see byte_times_128).
+TR_HD uint32_t byte_of(uint32_t w, int i)
 {
 #ifdef __CUDA_ARCH__
-    return __uint_as_float(__byte_perm(w, 0x4B00u, 0x5440u | uint32_t(i))) - 8388608.0f;
+    return __dp4a(w, 1u << (8 * i), 0u);
 #else
-    return float((w >> (8 * i)) & 0xffu);
+    return (w >> (8 * i)) & 0xffu;
+#endif
+}
+
+// 128 * (byte i of w). On the device one integer dot product, which leaves the ALU pipe (the
+// comparisons' pipe, the busiest of the quantized traversal) alone: byte permutes there, and
+// the add that they need, made the 1080p heightfield render 12 % slower.
+TR_HD uint32_t byte_times_128(uint32_t w, int i)
+{
+#ifdef __CUDA_ARCH__
+    return __dp4a(w, 128u << (8 * i), 0u);
+#else
+    return ((w >> (8 * i)) & 0xffu) << 7;
 #endif
 }
 
@@ -176,19 +196,11 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b)
-{
-    unsigned long long d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-// Byte j of lo and of hi, each placed in the low mantissa bits of 2^23.
+// byte_times_128 of byte j of a near and a far plane's word as a packed pair.
 __device__ __forceinline__ unsigned long long byte_pair(uint32_t lo, uint32_t hi, int j)
 {
-    const uint32_t a = __byte_perm(lo, 0x4B00u, 0x5440u | uint32_t(j));
-    const uint32_t b = __byte_perm(hi, 0x4B00u, 0x5440u | uint32_t(j));
     unsigned long long d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(a), "r"(b));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(byte_times_128(lo, j)), "r"(byte_times_128(hi, j)));
     return d;
 }
 __device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b)
@@ -217,6 +229,33 @@ __device__ __forceinline__ float min3(float a, float b, float c)
 }
 #endif
 
+// Bit i of the result is bit i ^ octInv of the low 8 bits of m: the children hit, by slot,
+// in the order the ray visits them (three conditional exchanges of neighbours).
+TR_HD uint32_t octant_order(uint32_t m, uint32_t octInv)
+{
+    if (octInv & 1u)
+        m = ((m << 1) & 0xaau) | ((m >> 1) & 0x55u);
+    if (octInv & 2u)
+        m = ((m << 2) & 0xccu) | ((m >> 2) & 0x33u);
+    if (octInv & 4u)
+        m = ((m << 4) & 0xf0u) | ((m >> 4) & 0x0fu);
+    return m;
+}
+
+// The hit mask of a node from the children hit (bit per slot), the internal children and the
+// meta bytes: bits 24..31 the internal children hit in the ray's octant order, bits 0..23 the
+// triangles of the leaves hit (few: their meta bytes are read one by one).
+TR_HD uint32_t hit_mask(uint32_t hits, uint32_t imask, uint32_t meta0, uint32_t meta1, uint32_t octInv)
+{
+    uint32_t tris = 0;
+    for (uint32_t leaves = hits & ~imask; leaves != 0u; leaves &= leaves - 1u) {
+        const uint32_t sl = ffs32(leaves) - 1u;
+        const uint32_t m = ((sl < 4u ? meta0 : meta1) >> (8u * (sl & 3u))) & 0xffu;
+        tris |= (m >> 5) << (m & 31u);
+    }
+    return (octant_order(hits & imask, octInv) << 24) | tris;
+}
+
 // Intersects the 8 children of a node; returns the hit mask: bits 24..31 for
 // internal children (position 24 + (slot ^ (7 - octant))), bits 0..23 for
 // leaf triangles (offset from the node's triangle base). imask gets the
@@ -241,28 +280,15 @@ TR_HD uint32_t intersect_wnode(const WideNode* __restrict__ nodes, uint32_t node
     const float* farY = ny ? node->lo[1] : node->hi[1];
     const float* nearZ = nz ? node->hi[2] : node->lo[2];
     const float* farZ = nz ? node->lo[2] : node->hi[2];
+    uint32_t miss = 0;  // bit per slot: the child is not hit
 #ifdef __CUDA_ARCH__
     const unsigned long long ox2 = pack2(O.x, O.x), oy2 = pack2(O.y, O.y), oz2 = pack2(O.z, O.z);
     const unsigned long long ix2 = pack2(invD.x, invD.x), iy2 = pack2(invD.y, invD.y), iz2 = pack2(invD.z, invD.z);
 #endif
-
-    // Per byte of meta: the hit-mask bit position (internal children, whose
-    // low five bits are >= 24, are re-ordered by the ray octant) and the bits
-    // to set there (the unary triangle count, or one bit for an internal
-    // child; zero for an empty slot, so empty slots need no branch).
-    const uint32_t octInv4 = octInv * 0x01010101u;
-    uint32_t hitmask = 0;
-    imask = 0;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const uint32_t meta4 = half == 0 ? h.z : h.w;
-        const uint32_t inner4 = ((meta4 & (meta4 << 1)) & 0x10101010u) >> 4;  // 1 per internal child
-        // the four 0/1 bytes gathered into bits 28..31 by one multiply
-        imask |= ((inner4 * 0x10204080u) >> 28) << (4 * half);
-        const uint32_t bitIndex4 = (meta4 ^ (octInv4 & (inner4 * 0xffu))) & 0x1f1f1f1fu;
-        const uint32_t childBits4 = (meta4 >> 5) & 0x07070707u;
-        float t0x[4], t1x[4], t0y[4], t1y[4], t0z[4], t1z[4];
+    for (int half = 1; half >= 0; --half) {
 #ifdef __CUDA_ARCH__
+        float t0x[4], t1x[4], t0y[4], t1y[4], t0z[4], t1z[4];
         const float4 nX = ldg(reinterpret_cast<const float4*>(nearX) + half);
         const float4 fX = ldg(reinterpret_cast<const float4*>(farX) + half);
         const float4 nY = ldg(reinterpret_cast<const float4*>(nearY) + half);
@@ -281,36 +307,36 @@ TR_HD uint32_t intersect_wnode(const WideNode* __restrict__ nodes, uint32_t node
         slab(fY, oy2, iy2, t1y);
         slab(nZ, oz2, iz2, t0z);
         slab(fZ, oz2, iz2, t1z);
-#else
-        for (int j = 0; j < 4; ++j) {
-            const int sl = 4 * half + j;
-            t0x[j] = mul_rn(sub_rn(nearX[sl], O.x), invD.x);
-            t1x[j] = mul_rn(sub_rn(farX[sl], O.x), invD.x);
-            t0y[j] = mul_rn(sub_rn(nearY[sl], O.y), invD.y);
-            t1y[j] = mul_rn(sub_rn(farY[sl], O.y), invD.y);
-            t0z[j] = mul_rn(sub_rn(nearZ[sl], O.z), invD.z);
-            t1z[j] = mul_rn(sub_rn(farZ[sl], O.z), invD.z);
-        }
-#endif
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-#ifdef __CUDA_ARCH__
+        for (int j = 3; j >= 0; --j) {
             const float tn = max3(t0x[j], t0y[j], fmaxf(t0z[j], tmin));
             const float tf = min3(t1x[j], t1y[j], fminf(t1z[j], tmax));
-#else
-            const float tn = fmaxf(fmaxf(t0x[j], t0y[j]), fmaxf(t0z[j], tmin));
-            const float tf = fminf(fminf(t1x[j], t1y[j]), fminf(t1z[j], tmax));
-#endif
-            if (tn <= tf * 1.0000004f)
-                hitmask |= ((childBits4 >> (8 * j)) & 7u) << ((bitIndex4 >> (8 * j)) & 31u);
+            // the sign of tf * 1.0000004 - tn
+            miss = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, 1.0000004f, -tn)), miss, 1);
         }
+#else
+        for (int j = 3; j >= 0; --j) {
+            const int sl = 4 * half + j;
+            const float t0x = mul_rn(sub_rn(nearX[sl], O.x), invD.x), t1x = mul_rn(sub_rn(farX[sl], O.x), invD.x);
+            const float t0y = mul_rn(sub_rn(nearY[sl], O.y), invD.y), t1y = mul_rn(sub_rn(farY[sl], O.y), invD.y);
+            const float t0z = mul_rn(sub_rn(nearZ[sl], O.z), invD.z), t1z = mul_rn(sub_rn(farZ[sl], O.z), invD.z);
+            const float tn = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, tmin));
+            const float tf = fminf(fminf(t1x, t1y), fminf(t1z, tmax));
+            miss = (miss << 1) | (std::signbit(fma_rn(tf, 1.0000004f, -tn)) ? 1u : 0u);
+        }
+#endif
     }
-    return hitmask;
+    // internal children: the meta bytes with bits 3 and 4 set, gathered to a bit per slot by
+    // one multiply a half
+    const uint32_t in0 = ((h.z & (h.z << 1)) & 0x10101010u) >> 4, in1 = ((h.w & (h.w << 1)) & 0x10101010u) >> 4;
+    imask = ((in0 * 0x10204080u) >> 28) | (((in1 * 0x10204080u) >> 24) & 0xf0u);
+    return hit_mask(~miss & 0xffu, imask, h.z, h.w, octInv);
 }
 
 // The same for a node with 8-bit quantized child boxes (the compressed wide BVH
 // of Ylitie et al.): a child plane is p + q * 2^e of the node's origin and
-// exponents, its distance one fused multiply-add of the byte.
+// exponents, its distance one fused multiply-add of the byte. invD and the test's time are
+// at kQuantTime.
 TR_HD uint32_t intersect_qnode(const QuantNode* __restrict__ nodes, uint32_t nodeIx,
                                                    const float3& O, const float3& invD, uint32_t octInv, float tmin,
                                                    float tmax, uint32_t& childBase, uint32_t& triBase,
@@ -324,19 +350,19 @@ TR_HD uint32_t intersect_qnode(const QuantNode* __restrict__ nodes, uint32_t nod
     const uint4 w4 = ldg(nw + 4);
 
     const float px = u2f(w0.x), py = u2f(w0.y), pz = u2f(w0.z);
-    const float sx = u2f((w0.w & 0xffu) << 23);
-    const float sy = u2f(((w0.w >> 8) & 0xffu) << 23);
-    const float sz = u2f(((w0.w >> 16) & 0xffu) << 23);
     imask = w0.w >> 24;
     childBase = w1.x;
     triBase = w1.y;
 
-    const float ax = sx * invD.x, ay = sy * invD.y, az = sz * invD.z;
+    // a step's distance times 2^142: the step's exponent added to the reciprocal direction's
+    const float ax = u2f(f2u(invD.x) + (byte_of(w0.w, 0) << 23));
+    const float ay = u2f(f2u(invD.y) + (byte_of(w0.w, 1) << 23));
+    const float az = u2f(f2u(invD.z) + (byte_of(w0.w, 2) << 23));
     const float bx = (px - O.x) * invD.x, by = (py - O.y) * invD.y, bz = (pz - O.z) * invD.z;
+    const float tlo = tmin * kQuantTime, thi = tmax * kQuantTime;
 #ifdef __CUDA_ARCH__
     const unsigned long long ax2 = pack2(ax, ax), ay2 = pack2(ay, ay), az2 = pack2(az, az);
     const unsigned long long bx2 = pack2(bx, bx), by2 = pack2(by, by), bz2 = pack2(bz, bz);
-    const unsigned long long kMinus2p23x2 = pack2(-8388608.0f, -8388608.0f);
 #endif
 
     // octant swizzle: the near plane is qhi on axes the ray walks backwards
@@ -348,47 +374,40 @@ TR_HD uint32_t intersect_qnode(const QuantNode* __restrict__ nodes, uint32_t nod
     const uint32_t loZ0 = nz ? w4.z : w3.x, loZ1 = nz ? w4.w : w3.y;
     const uint32_t hiZ0 = nz ? w3.x : w4.z, hiZ1 = nz ? w3.y : w4.w;
 
-    // Per byte of meta: the hit-mask bit position (internal children, whose
-    // low five bits are >= 24, are re-ordered by the ray octant) and the bits
-    // to set there (the unary triangle count, or one bit for an internal
-    // child; zero for an empty slot, so empty slots need no branch).
-    const uint32_t octInv4 = octInv * 0x01010101u;
-    uint32_t hitmask = 0;
+    uint32_t miss = 0;  // bit per slot: the child is not hit
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-        const uint32_t meta4 = half == 0 ? w1.z : w1.w;
-        const uint32_t inner4 = ((meta4 & (meta4 << 1)) & 0x10101010u) >> 4;  // 1 per internal child
-        const uint32_t bitIndex4 = (meta4 ^ (octInv4 & (inner4 * 0xffu))) & 0x1f1f1f1fu;
-        const uint32_t childBits4 = (meta4 >> 5) & 0x07070707u;
+    for (int half = 1; half >= 0; --half) {
         const uint32_t lx = half == 0 ? loX0 : loX1, hx = half == 0 ? hiX0 : hiX1;
         const uint32_t ly = half == 0 ? loY0 : loY1, hy = half == 0 ? hiY0 : hiY1;
         const uint32_t lz = half == 0 ? loZ0 : loZ1, hz = half == 0 ? hiZ0 : hiZ1;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 3; j >= 0; --j) {
 #ifdef __CUDA_ARCH__
-            // near and far plane of an axis as one packed pair: two byte permutes, one
-            // packed add, one packed FMA (each lane rounds as the scalar fma_rn does)
+            // near and far plane of an axis as one packed pair: two integer dot products and
+            // one packed FMA (each lane rounds as the scalar fma_rn does)
             float t0x, t1x, t0y, t1y, t0z, t1z;
-            unpack2(fma2(add2(byte_pair(lx, hx, j), kMinus2p23x2), ax2, bx2), t0x, t1x);
-            unpack2(fma2(add2(byte_pair(ly, hy, j), kMinus2p23x2), ay2, by2), t0y, t1y);
-            unpack2(fma2(add2(byte_pair(lz, hz, j), kMinus2p23x2), az2, bz2), t0z, t1z);
-            const float tn = max3(t0x, t0y, fmaxf(t0z, tmin));
-            const float tf = min3(t1x, t1y, fminf(t1z, tmax));
+            unpack2(fma2(byte_pair(lx, hx, j), ax2, bx2), t0x, t1x);
+            unpack2(fma2(byte_pair(ly, hy, j), ay2, by2), t0y, t1y);
+            unpack2(fma2(byte_pair(lz, hz, j), az2, bz2), t0z, t1z);
+            const float tn = max3(t0x, t0y, fmaxf(t0z, tlo));
+            const float tf = min3(t1x, t1y, fminf(t1z, thi));
+            // the sign of tf * 1.0000004 - tn
+            miss = __funnelshift_l(__float_as_uint(__fmaf_rn(tf, 1.0000004f, -tn)), miss, 1);
 #else
-            const float t0x = fma_rn(byte_to_float(lx, j), ax, bx);
-            const float t1x = fma_rn(byte_to_float(hx, j), ax, bx);
-            const float t0y = fma_rn(byte_to_float(ly, j), ay, by);
-            const float t1y = fma_rn(byte_to_float(hy, j), ay, by);
-            const float t0z = fma_rn(byte_to_float(lz, j), az, bz);
-            const float t1z = fma_rn(byte_to_float(hz, j), az, bz);
-            const float tn = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, tmin));
-            const float tf = fminf(fminf(t1x, t1y), fminf(t1z, tmax));
+            const float t0x = fma_rn(u2f(byte_times_128(lx, j)), ax, bx);
+            const float t1x = fma_rn(u2f(byte_times_128(hx, j)), ax, bx);
+            const float t0y = fma_rn(u2f(byte_times_128(ly, j)), ay, by);
+            const float t1y = fma_rn(u2f(byte_times_128(hy, j)), ay, by);
+            const float t0z = fma_rn(u2f(byte_times_128(lz, j)), az, bz);
+            const float t1z = fma_rn(u2f(byte_times_128(hz, j)), az, bz);
+            const float tn = fmaxf(fmaxf(t0x, t0y), fmaxf(t0z, tlo));
+            const float tf = fminf(fminf(t1x, t1y), fminf(t1z, thi));
+            miss = (miss << 1) | (std::signbit(fma_rn(tf, 1.0000004f, -tn)) ? 1u : 0u);
 #endif
-            if (tn <= tf * 1.0000004f)
-                hitmask |= ((childBits4 >> (8 * j)) & 7u) << ((bitIndex4 >> (8 * j)) & 31u);
         }
     }
-    return hitmask;
+    // (an empty slot's box is not empty, but its meta byte sets no triangle)
+    return hit_mask(~miss & 0xffu, imask, w1.z, w1.w, octInv);
 }
 
 // Resumable traversal state of one ray: the persistent extend/connect kernels
@@ -397,7 +416,6 @@ struct Traversal {
     float3 O;
     float3 D;
     float3 invD;
-    float tmin;
     float tmax;
     float u;
     float v;
@@ -409,17 +427,27 @@ struct Traversal {
     bool ok;
 };
 
-TR_HD void traversal_begin(Traversal& t, const float3& O, const float3& D, float tmin, float tmax, uint32_t root = 0)
+// Node layout a traversal is compiled for: fp32 or quantized child boxes.
+enum : int { kLayoutWide = 1, kLayoutQuant = 2 };
+
+template <int LAYOUT>
+TR_HD void set_ray(Traversal& t, const float3& O, const float3& D)
 {
     const float kTiny = 1e-20f;
     t.O = O;
     t.D = D;
-    t.invD = make_float3(1.0f / (fabsf(D.x) > kTiny ? D.x : copysignf(kTiny, D.x)),
-                         1.0f / (fabsf(D.y) > kTiny ? D.y : copysignf(kTiny, D.y)),
-                         1.0f / (fabsf(D.z) > kTiny ? D.z : copysignf(kTiny, D.z)));
+    const float scale = LAYOUT == kLayoutQuant ? kQuantTime : 1.0f;
+    t.invD = make_float3(1.0f / (fabsf(D.x) > kTiny ? D.x : copysignf(kTiny, D.x)) * scale,
+                         1.0f / (fabsf(D.y) > kTiny ? D.y : copysignf(kTiny, D.y)) * scale,
+                         1.0f / (fabsf(D.z) > kTiny ? D.z : copysignf(kTiny, D.z)) * scale);
     const uint32_t octant = (t.invD.x < 0.f ? 1u : 0u) | (t.invD.y < 0.f ? 2u : 0u) | (t.invD.z < 0.f ? 4u : 0u);
     t.octInv = 7u - octant;
-    t.tmin = tmin;
+}
+
+template <int LAYOUT>
+TR_HD void traversal_begin(Traversal& t, const float3& O, const float3& D, float tmax, uint32_t root = 0)
+{
+    set_ray<LAYOUT>(t, O, D);
     t.tmax = tmax;
     t.u = 0.f;
     t.v = 0.f;
@@ -438,12 +466,8 @@ TR_HD void traversal_begin(Traversal& t, const float3& O, const float3& D, float
 // becomes its internal children (the rest of the old group waits on the
 // stack); returns its leaf group (base, bits). Returns false when a bound ran
 // out (t.ok cleared).
-// Node layout a traversal is compiled for: the scene's (a uniform branch per
-// node on SceneView::quantNodes), or fixed to fp32 or quantized child boxes.
-enum : int { kLayoutScene = 0, kLayoutWide = 1, kLayoutQuant = 2 };
-
-template <bool COUNT, int LAYOUT = kLayoutScene>
-TR_HD bool node_step(Traversal& t, uint2* stack, const void* __restrict__ nodes, bool quant, uint32_t stepLimit,
+template <bool COUNT, int LAYOUT>
+TR_HD bool node_step(Traversal& t, float tmin, uint2* stack, const void* __restrict__ nodes, uint32_t stepLimit,
                      TraversalCounts* cnt, uint2& leaves)
 {
     leaves = make_uint2(0u, 0u);
@@ -462,14 +486,12 @@ TR_HD bool node_step(Traversal& t, uint2* stack, const void* __restrict__ nodes,
             t.ok = false;
     }
     uint32_t childBase, triBase, imask;
-    // the node layout is the same for every ray of a launch (a uniform branch
-    // when it is not fixed at compile time)
-    const bool q = LAYOUT == kLayoutQuant || (LAYOUT == kLayoutScene && quant);
     const uint32_t hm =
-        q ? intersect_qnode(static_cast<const QuantNode*>(nodes), nodeIx, t.O, t.invD, t.octInv, t.tmin, t.tmax,
-                                childBase, triBase, imask)
-              : intersect_wnode(static_cast<const WideNode*>(nodes), nodeIx, t.O, t.invD, t.octInv, t.tmin, t.tmax,
-                                childBase, triBase, imask);
+        LAYOUT == kLayoutQuant
+            ? intersect_qnode(static_cast<const QuantNode*>(nodes), nodeIx, t.O, t.invD, t.octInv, tmin, t.tmax,
+                              childBase, triBase, imask)
+            : intersect_wnode(static_cast<const WideNode*>(nodes), nodeIx, t.O, t.invD, t.octInv, tmin, t.tmax,
+                              childBase, triBase, imask);
     if (COUNT)
         cnt->nodes++;
     t.group = make_uint2(childBase, (hm & 0xff000000u) | imask);
@@ -485,14 +507,14 @@ TR_HD bool node_step(Traversal& t, uint2* stack, const void* __restrict__ nodes,
 // its hit, 1 when a closer hit was recorded, 0 otherwise. PAIR (closest hit
 // only) fetches two triangles before testing either.
 template <bool ANY, bool COUNT, bool PAIR = false>
-TR_HD int leaf_triangles(Traversal& t, uint2 tris, const SceneView& s, TraversalCounts* cnt)
+TR_HD int leaf_triangles(Traversal& t, float tmin, uint2 tris, const SceneView& s, TraversalCounts* cnt)
 {
     int found = 0;
     auto test = [&](uint32_t slot, const float4& a, const float4& b, const float4& c) -> bool {
         if (COUNT)
             cnt->tris++;
         float tt, uu, vv;
-        if (intersect_triangle(t.O, t.D, a, b, c, t.tmin, t.tmax, tt, uu, vv)) {
+        if (intersect_triangle(t.O, t.D, a, b, c, tmin, t.tmax, tt, uu, vv)) {
             if (ANY) {
                 t.tmax = tt;
                 t.hitSlot = slot;
@@ -546,27 +568,13 @@ TR_HD int leaf_triangles(Traversal& t, uint2 tris, const SceneView& s, Traversal
 // triangles it reports, then a stack pop if the group is exhausted. Returns
 // true when the ray is finished (t.hitSlot, t.tmax, t.u, t.v hold the result;
 // t.ok is false if a bound was exceeded).
-template <bool ANY, bool COUNT, int LAYOUT = kLayoutScene>
-TR_HD bool traversal_step(Traversal& t, uint2* stack, const SceneView& s, TraversalCounts* cnt)
+template <bool ANY, bool COUNT, int LAYOUT>
+TR_HD bool traversal_step(Traversal& t, float tmin, uint2* stack, const SceneView& s, TraversalCounts* cnt)
 {
     uint2 tris;
-    if (!node_step<COUNT, LAYOUT>(t, stack, s.nodes, s.quantNodes != 0, s.stepLimit, cnt, tris))
+    if (!node_step<COUNT, LAYOUT>(t, tmin, stack, s.nodes, s.stepLimit, cnt, tris))
         return true;
-#ifdef __CUDA_ARCH__
-    // closest hit: the next node (the first hit child of the new group) into L1
-    // while the leaf triangles are tested (extend 51.9 -> 51.6 ms per 1080p,
-    // 64 spp heightfield step; shadow rays lost 0.4 ms with it)
-    if (!ANY && LAYOUT == kLayoutWide && tris.y != 0u && t.group.y > 0x00ffffffu) {
-        const uint32_t hits = t.group.y;
-        const uint32_t slot = (31u - clz32(hits) - 24u) ^ t.octInv;
-        const uint32_t next = t.group.x + popc32(hits & 0xffu & ((1u << slot) - 1u));
-        const char* a = reinterpret_cast<const char*>(static_cast<const WideNode*>(s.nodes) + next);
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 128));
-        asm volatile("prefetch.global.L1 [%0];" ::"l"(a + 192));
-    }
-#endif
-    if (leaf_triangles<ANY, COUNT, !ANY>(t, tris, s, cnt) == 2)
+    if (leaf_triangles<ANY, COUNT, !ANY>(t, tmin, tris, s, cnt) == 2)
         return true;
     if (t.group.y <= 0x00ffffffu) {
         if (t.sp == 0)
@@ -592,18 +600,6 @@ TR_HD float3 xform_vector(const float4& r0, const float4& r1, const float4& r2, 
                        add_rn(add_rn(mul_rn(r2.x, v.x), mul_rn(r2.y, v.y)), mul_rn(r2.z, v.z)));
 }
 
-TR_HD void set_ray(Traversal& t, const float3& O, const float3& D)
-{
-    const float kTiny = 1e-20f;
-    t.O = O;
-    t.D = D;
-    t.invD = make_float3(1.0f / (fabsf(D.x) > kTiny ? D.x : copysignf(kTiny, D.x)),
-                         1.0f / (fabsf(D.y) > kTiny ? D.y : copysignf(kTiny, D.y)),
-                         1.0f / (fabsf(D.z) > kTiny ? D.z : copysignf(kTiny, D.z)));
-    const uint32_t octant = (t.invD.x < 0.f ? 1u : 0u) | (t.invD.y < 0.f ? 2u : 0u) | (t.invD.z < 0.f ? 4u : 0u);
-    t.octInv = 7u - octant;
-}
-
 // Two-level traversal (the instance BVH, then the BVH of each instance's mesh
 // in object space; replaces OptiX's instance acceleration structure). The
 // object-space ray keeps the world ray's parameter t, so t and tmax compare
@@ -620,9 +616,10 @@ struct TraversalTL {
     uint32_t hitInst;     // instance of the recorded hit
 };
 
-TR_HD void traversal_begin(TraversalTL& r, const float3& O, const float3& D, float tmin, float tmax, uint32_t = 0)
+template <int LAYOUT>
+TR_HD void traversal_begin(TraversalTL& r, const float3& O, const float3& D, float tmax, uint32_t = 0)
 {
-    traversal_begin(r.t, O, D, tmin, tmax, 0u);
+    traversal_begin<LAYOUT>(r.t, O, D, tmax, 0u);
     r.wO = O;
     r.wD = D;
     r.wInvD = r.t.invD;
@@ -634,8 +631,8 @@ TR_HD void traversal_begin(TraversalTL& r, const float3& O, const float3& D, flo
 }
 
 // (two levels: the instance BVH has the layout of the mesh BVHs)
-template <bool ANY, bool COUNT, int LAYOUT = kLayoutScene>
-TR_HD bool traversal_step(TraversalTL& r, uint2* stack, const SceneView& s, TraversalCounts* cnt)
+template <bool ANY, bool COUNT, int LAYOUT>
+TR_HD bool traversal_step(TraversalTL& r, float tmin, uint2* stack, const SceneView& s, TraversalCounts* cnt)
 {
     Traversal& t = r.t;
     if (r.inst == kNoInstance && r.leafGroup.y != 0u) {
@@ -657,7 +654,7 @@ TR_HD bool traversal_step(TraversalTL& r, uint2* stack, const SceneView& s, Trav
         const float4 r0 = ldg(s.invTransforms + 3u * id + 0u);
         const float4 r1 = ldg(s.invTransforms + 3u * id + 1u);
         const float4 r2 = ldg(s.invTransforms + 3u * id + 2u);
-        set_ray(t, xform_point(r0, r1, r2, r.wO), xform_vector(r0, r1, r2, r.wD));
+        set_ray<LAYOUT>(t, xform_point(r0, r1, r2, r.wO), xform_vector(r0, r1, r2, r.wD));
         r.inst = id;
         r.instSp = t.sp;
         t.group = make_uint2(ldg(&s.instInfo[id].x), 0x80000000u);
@@ -669,13 +666,12 @@ TR_HD bool traversal_step(TraversalTL& r, uint2* stack, const SceneView& s, Trav
     }
     const bool top = r.inst == kNoInstance;
     uint2 leaves;
-    if (!node_step<COUNT, LAYOUT>(t, stack, top ? s.tlasNodes : s.nodes, s.quantNodes != 0, s.stepLimit, cnt,
-                                  leaves))
+    if (!node_step<COUNT, LAYOUT>(t, tmin, stack, top ? s.tlasNodes : s.nodes, s.stepLimit, cnt, leaves))
         return true;
     if (top) {
         r.leafGroup = leaves;  // entered one by one in the next steps
     } else {
-        const int found = leaf_triangles<ANY, COUNT>(t, leaves, s, cnt);
+        const int found = leaf_triangles<ANY, COUNT>(t, tmin, leaves, s, cnt);
         if (found)
             r.hitInst = r.inst;
         if (found == 2)
@@ -727,35 +723,39 @@ TR_HD uint32_t hit_instance(const TraversalTL& r) { return r.hitInst; }
 // ANY = true stops at the first hit inside [tmin, tmax]. Returns false when a
 // bound (stack depth, step count) was exceeded; the hit reported so far is
 // kept. COUNT adds the nodes and triangles visited to *cnt.
+template <bool ANY, bool COUNT, bool TL, int LAYOUT>
+TR_HD bool traverse_layout(const SceneView& s, const float3& O, const float3& D, float tmin, float& tmax,
+                           uint32_t& hitSlot, float& hu, float& hv, TraversalCounts* cnt, uint32_t& hitInst)
+{
+    uint2 stack[kTraversalStack];
+    typename TravOf<TL>::type r;
+    traversal_begin<LAYOUT>(r, O, D, tmax);
+    while (!traversal_step<ANY, COUNT, LAYOUT>(r, tmin, stack, s, cnt)) {
+    }
+    tmax = base(r).tmax;
+    hitSlot = base(r).hitSlot;
+    hu = base(r).u;
+    hv = base(r).v;
+    hitInst = hit_instance(r);
+    return base(r).ok;
+}
+
 template <bool ANY, bool COUNT = false>
 TR_HD bool traverse(const SceneView& s, const float3& O, const float3& D, float tmin, float& tmax, uint32_t& hitSlot,
                     float& hu, float& hv, TraversalCounts* cnt = nullptr, uint32_t* hitInst = nullptr)
 {
-    uint2 stack[kTraversalStack];
-    if (s.tlasNodes) {
-        TraversalTL r;
-        traversal_begin(r, O, D, tmin, tmax);
-        while (!traversal_step<ANY, COUNT>(r, stack, s, cnt)) {
-        }
-        tmax = r.t.tmax;
-        hitSlot = r.t.hitSlot;
-        hu = r.t.u;
-        hv = r.t.v;
-        if (hitInst)
-            *hitInst = r.hitInst;
-        return r.t.ok;
-    }
-    Traversal t;
-    traversal_begin(t, O, D, tmin, tmax);
-    while (!traversal_step<ANY, COUNT>(t, stack, s, cnt)) {
-    }
-    tmax = t.tmax;
-    hitSlot = t.hitSlot;
-    hu = t.u;
-    hv = t.v;
+    uint32_t inst = 0u;
+    const bool ok =
+        s.tlasNodes
+            ? (s.quantNodes
+                   ? traverse_layout<ANY, COUNT, true, kLayoutQuant>(s, O, D, tmin, tmax, hitSlot, hu, hv, cnt, inst)
+                   : traverse_layout<ANY, COUNT, true, kLayoutWide>(s, O, D, tmin, tmax, hitSlot, hu, hv, cnt, inst))
+            : (s.quantNodes
+                   ? traverse_layout<ANY, COUNT, false, kLayoutQuant>(s, O, D, tmin, tmax, hitSlot, hu, hv, cnt, inst)
+                   : traverse_layout<ANY, COUNT, false, kLayoutWide>(s, O, D, tmin, tmax, hitSlot, hu, hv, cnt, inst));
     if (hitInst)
-        *hitInst = 0u;
-    return t.ok;
+        *hitInst = inst;
+    return ok;
 }
 
 } // namespace tr
