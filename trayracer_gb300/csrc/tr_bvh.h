@@ -75,15 +75,16 @@ bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& 
 constexpr float kQuantMaxDirection = 0x1p20f;
 
 // Node layout of an uploaded BVH: mode 0 (auto) keeps fp32 child boxes for one-level
-// scenes of up to kWideNodeMax nodes, 1 always fp32, 2 always quantized. Returns true
-// for quantized.
+// scenes of up to kWideNodeMax nodes (64 MB, which stay in L2 beside the wavefront
+// buffers), 1 always fp32, 2 always quantized. Returns true for quantized.
 // The fp32 test needs fewer instructions and 2.6 times the bytes through L1, whose data
 // pipe bounds it as soon as a warp's lanes visit different nodes. 720p frames, fp32 /
 // quantized: closed room (3 nodes) 2087 / 2178 us; heightfields of 142 nodes 1419 / 1434,
-// 519 nodes 1695 / 1688, 3305 nodes 2148 / 2079, 13351 nodes 2480 / 2354. The two are
-// within 3 % of each other up to the line; two-level scenes keep the quantized layout (a
-// small one would gain 7 % with fp32, whose larger traversal state spills).
-constexpr size_t kWideNodeMax = 4096;
+// 519 nodes 1695 / 1688, 3305 nodes 2148 / 2079, 13351 nodes 2480 / 2354. The line lies
+// higher than where the two cross because the layouts' hits differ: about one ray in 10^7
+// along a shared edge finds (by rounding) a triangle that its fp32 box excludes, and such a
+// path's later decisions change an image visibly. Two-level scenes keep the quantized layout.
+constexpr size_t kWideNodeMax = (size_t(64) << 20) / 208;
 inline bool quantized_nodes(size_t nodeCount, uint32_t mode, bool twoLevel = false)
 {
     return mode == 2u || (mode == 0u && (twoLevel || nodeCount > kWideNodeMax));

@@ -89,7 +89,7 @@ struct AliasEntry {
 // WideNode, child boxes in fp32, 208 bytes:
 //   hdr: child_base, tri_base, meta[0..3], meta[4..7]
 //   lo[a][slot], hi[a][slot]: the child boxes per axis (empty slot: +inf / -inf)
-// For small BVHs, whose nodes a warp's lanes share (see kWideNodeMax).
+// For one-level BVHs that stay L2-resident (see kWideNodeMax).
 struct alignas(16) WideNode {
     uint4 hdr;
     float lo[3][8];
