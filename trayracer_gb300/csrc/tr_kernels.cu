@@ -408,6 +408,92 @@ constexpr uint32_t kRefillBelow = 10;
 // Largest block of the persistent traversal kernels (LaunchShape::traversalThreads).
 constexpr uint32_t kTraversalThreadsMax = 128;
 
+// Triangle tests of a warp's shadow rays (one-level scenes). A step leaves leaf triangles with a
+// few of the warp's lanes only (3.4 of 17 on a heightfield, 1.7 times a step), and a test for
+// them costs as much as one for 32 rays. The lanes therefore list their triangles, and the warp
+// tests the listed ones together, one a lane, against the owner's ray kept here. Heightfield
+// render (1080p, 64 spp) 91.8 -> 88.4 ms with fp32 nodes, 87.8 -> 83.2 ms with quantized ones.
+// (Closest-hit rays lose with it, 83.2 -> 87.9 ms: what a test finds has to travel back to the
+// owner, and nodes are visited that the hit would cull.)
+struct WarpTriangles {
+    float4 O[32];      // origin, tmax
+    float4 D[32];
+    uint2 entry[32];   // triangle slot, owner lane
+};
+// Listed triangles from which the warp tests them at once; fewer wait for more while enough
+// lanes have nodes to visit (16 and 24 within 0.1 %, 8 and 32 1 %, at once 3 % slower).
+constexpr uint32_t kTriangleBatch = 16;
+
+// Tests the listed triangles (count of them); `mine` has a bit for each entry of this lane.
+template <bool COUNT>
+__device__ __forceinline__ void test_listed(Traversal& t, WarpTriangles& w, float tmin, const SceneView& s,
+                                            uint32_t& count, uint32_t& mine, TraversalCounts* cnt)
+{
+    const uint32_t lane = lane_id();
+    __syncwarp();
+    bool hit = false;
+    if (lane < count) {
+        const uint2 e = w.entry[lane];
+        const float4 o = w.O[e.y], d = w.D[e.y];
+        const float4* tp = s.bvhTris + 3u * e.x;
+        float tt, uu, vv;
+        hit = intersect_triangle(f3(o), f3(d), __ldg(tp + 0), __ldg(tp + 1), __ldg(tp + 2), tmin, o.w, tt, uu, vv);
+        if (COUNT)
+            cnt->tris++;
+    }
+    if (__ballot_sync(kFull, hit) & mine)
+        t.hitSlot = 0u;
+    mine = 0u;
+    count = 0u;
+    __syncwarp();
+}
+
+// Visits nodes with the warp's shadow rays until fewer than `below` of them are alive; the rays
+// that end set `ended` (t.hitSlot other than ~0: occluded).
+template <bool COUNT, int LAYOUT>
+__device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles& w, uint2* stack, const SceneView& s,
+                                              float tmin, uint32_t below, bool& alive, bool& ended,
+                                              TraversalCounts* cnt)
+{
+    const uint32_t lane = lane_id();
+    uint32_t count = 0, mine = 0, active;
+    do {
+        uint2 tris = make_uint2(0u, 0u);
+        if (alive && t.group.y > 0x00ffffffu) {
+            if (!node_step<COUNT, LAYOUT>(t, tmin, stack, s.nodes, s.stepLimit, cnt, tris)) {
+                tris.y = 0u;  // out of steps: what is listed is still tested
+                t.group.y = 0u;
+                t.sp = 0;
+            } else if (t.group.y <= 0x00ffffffu && t.sp > 0) {
+                t.group = stack[--t.sp];
+            }
+        }
+        for (uint32_t m = __ballot_sync(kFull, tris.y != 0u); m != 0u; m = __ballot_sync(kFull, tris.y != 0u)) {
+            const uint32_t n = __popc(m);
+            if (count + n > 32u)
+                test_listed<COUNT>(t, w, tmin, s, count, mine, cnt);
+            if (tris.y != 0u) {
+                const uint32_t at = count + __popc(m & ((1u << lane) - 1u));
+                w.entry[at] = make_uint2(tris.x + __ffs(tris.y) - 1u, lane);
+                mine |= 1u << at;
+                tris.y &= tris.y - 1u;
+            }
+            count += n;
+        }
+        if (count >= kTriangleBatch ||
+            (count && __popc(__ballot_sync(kFull, alive && t.group.y > 0x00ffffffu)) < below))
+            test_listed<COUNT>(t, w, tmin, s, count, mine, cnt);
+        if (alive && (t.hitSlot != 0xffffffffu || (mine == 0u && t.group.y <= 0x00ffffffu))) {
+            alive = false;
+            ended = true;
+        }
+        active = __ballot_sync(kFull, alive);
+    } while (uint32_t(__popc(active)) >= below);
+    // (rays that ended leave their lanes to others: nothing of theirs stays listed)
+    if (count)
+        test_listed<COUNT>(t, w, tmin, s, count, mine, cnt);
+}
+
 // Closest hit of the bounce's extend queue. Rays that hit are appended (one
 // warp ballot and one atomic per step) to the hit queue with their full path
 // state and hit record; missed rays end here. COUNT = true also sums the nodes
@@ -1165,12 +1251,12 @@ __global__ void __launch_bounds__(256) sort_scatter_kernel(FrameView f, SortView
 // Any hit of the bounce's shadow queue over [eps, dist - 2 eps]; an unoccluded
 // ray adds its radiance to its path. Same lane refill as extend_kernel.
 // Blocks of 64 or 128 threads (LaunchShape::traversalThreads): the kernel works per warp.
-// One-level scenes: 56 registers, 9 blocks of 128 threads per SM (the kernel is bound by
-// the latency of its node fetches; 31.3 against 33.1 ms of shadow rays per 1080p, 64 spp
-// heightfield step at 72 registers and 7 blocks). Two-level traversal holds more state and
-// keeps its own register count (it would spill 100-210 bytes at 56).
+// One-level scenes: 56 registers, 9 blocks of 128 threads per SM (heightfield render 83.3 ms
+// against 83.9 at 8 blocks and 87.0 at 10). Two-level traversal holds more state: 7 blocks
+// (72 registers, 24 B spilled; 1024 x 768 frame of the two-level room 2642 us against 2681 at
+// 6 blocks and 2845 unbounded at 4, and it would spill 100-210 bytes at 9).
 template <bool COUNT, bool BATCH, bool TL, int LAYOUT>
-__global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, FrameView f, Settings st,
+__global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, FrameView f, Settings st,
                                                                    uint32_t bounce)
 {
     const uint32_t count = BATCH ? __ldcg(&f.batch->connectQueue) : __ldcg(f.counters + kShadowCounterBase + bounce);
@@ -1182,6 +1268,7 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
     __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
+    __shared__ WarpTriangles warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
     bool alive = false, ended = false, more = true;
     while (true) {
         // The rays that ended since the last refill, all lanes at once: the contribution of
@@ -1214,6 +1301,10 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
                 const uint32_t root =
                     BATCH ? __float_as_uint(__ldcs(reinterpret_cast<const float*>(f.shadow + i + 2 * cap) + 3)) : 0u;
                 traversal_begin<LAYOUT>(t, f3(O4), f3(L4), L4.w - (2 * st.rayEpsilon), root);
+                if (!TL) {
+                    warpTris[threadIdx.x >> 5].O[lane] = f4(f3(O4), L4.w - (2 * st.rayEpsilon));
+                    warpTris[threadIdx.x >> 5].D[lane] = L4;
+                }
                 alive = true;
             }
             more = first + __popc(idle) < count;
@@ -1222,14 +1313,19 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) connect_kernel(SceneView s, F
             break;
         // with the queue empty there is nothing to refill: the warp's rays run out together
         const uint32_t below = more ? st.refillBelow : 1u;
-        uint32_t active;
-        do {
-            if (alive && traversal_step<true, COUNT, LAYOUT>(t, st.rayEpsilon, stack, s, &cnt)) {
-                alive = false;
-                ended = true;
-            }
-            active = __ballot_sync(kFull, alive);
-        } while (uint32_t(__popc(active)) >= below);
+        if constexpr (TL) {
+            uint32_t active;
+            do {
+                if (alive && traversal_step<true, COUNT, LAYOUT>(t, st.rayEpsilon, stack, s, &cnt)) {
+                    alive = false;
+                    ended = true;
+                }
+                active = __ballot_sync(kFull, alive);
+            } while (uint32_t(__popc(active)) >= below);
+        } else {
+            trace_shadows<COUNT, LAYOUT>(t, warpTris[threadIdx.x >> 5], stack, s, st.rayEpsilon, below, alive, ended,
+                                         &cnt);
+        }
     }
     if (COUNT) {
         add_counts(f.traversal + 2, cnt);
@@ -1854,7 +1950,7 @@ __global__ void __launch_bounds__(kAdjointThreads, 4) adjoint_shade_kernel(Scene
 // takes its contribution off the path's remaining radiance and is listed for
 // nee_grad_kernel.
 template <bool TL, int LAYOUT>
-__global__ void __launch_bounds__(128, TL ? 1 : 9) adjoint_connect_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
+__global__ void __launch_bounds__(128, TL ? 7 : 9) adjoint_connect_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
                                                               AdjointView a)
 {
     const uint32_t count = __ldcg(f.counters + kShadowCounterBase + bounce);
@@ -1865,6 +1961,7 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) adjoint_connect_kernel(SceneV
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
     __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
+    __shared__ WarpTriangles warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
     bool alive = false, ended = false, more = true;
     while (true) {
         // the rays that ended since the last refill, all lanes at once (as connect_kernel)
@@ -1899,6 +1996,10 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) adjoint_connect_kernel(SceneV
                 const float4 L4 = __ldcs(f.shadow + i + cap);
                 rayIds[threadIdx.x] = make_uint2(i, __float_as_uint(O4.w));
                 traversal_begin<LAYOUT>(t, f3(O4), f3(L4), L4.w - (2 * st.rayEpsilon));
+                if (!TL) {
+                    warpTris[threadIdx.x >> 5].O[lane] = f4(f3(O4), L4.w - (2 * st.rayEpsilon));
+                    warpTris[threadIdx.x >> 5].D[lane] = L4;
+                }
                 alive = true;
             }
             more = first + __popc(idle) < count;
@@ -1906,14 +2007,19 @@ __global__ void __launch_bounds__(128, TL ? 1 : 9) adjoint_connect_kernel(SceneV
         if (!__any_sync(kFull, alive))
             break;
         const uint32_t below = more ? st.refillBelow : 1u;
-        uint32_t active;
-        do {
-            if (alive && traversal_step<true, false, LAYOUT>(t, st.rayEpsilon, stack, s, nullptr)) {
-                alive = false;
-                ended = true;
-            }
-            active = __ballot_sync(kFull, alive);
-        } while (uint32_t(__popc(active)) >= below);
+        if constexpr (TL) {
+            uint32_t active;
+            do {
+                if (alive && traversal_step<true, false, LAYOUT>(t, st.rayEpsilon, stack, s, nullptr)) {
+                    alive = false;
+                    ended = true;
+                }
+                active = __ballot_sync(kFull, alive);
+            } while (uint32_t(__popc(active)) >= below);
+        } else {
+            trace_shadows<false, LAYOUT>(t, warpTris[threadIdx.x >> 5], stack, s, st.rayEpsilon, below, alive, ended,
+                                         nullptr);
+        }
     }
 }
 
