@@ -132,6 +132,7 @@ struct Context {
     // b + 1's extend rays run on the frame's stream (fork / join)
     cudaStream_t side = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
+    cudaEvent_t evSummed = nullptr;    // tr_adjoint_frame: a bounce's light gradients are summed
     cudaEvent_t evExtend[TR_MAX_DEPTH] = {}, evShade[TR_MAX_DEPTH] = {}, evConnect[TR_MAX_DEPTH] = {};
     bool timedFrame = false;
     uint32_t timedDepth = 0;
@@ -684,7 +685,8 @@ tr_status tr_create(const tr_config* config, void** out_ctx)
     bool ok = cudaStreamCreate(&c->stream) == cudaSuccess;
     ok = ok && cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&c->evFork, cudaEventDisableTiming) == cudaSuccess &&
-         cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) == cudaSuccess;
+         cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) == cudaSuccess &&
+         cudaEventCreateWithFlags(&c->evSummed, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreate(&c->evStart) == cudaSuccess && cudaEventCreate(&c->evGenerate) == cudaSuccess &&
          cudaEventCreate(&c->evFinal) == cudaSuccess;
     for (uint32_t i = 0; ok && i < TR_MAX_DEPTH; ++i)
@@ -714,7 +716,8 @@ tr_status tr_destroy(void* ctx)
     c->adjointArena.release();
     c->samplesArena.release();
     release_textures(c);
-    cudaEvent_t* evs[] = {&c->evStart, &c->evGenerate, &c->evFinal, &c->evFork, &c->evJoin};
+    cudaEvent_t* evs[] = {&c->evStart, &c->evGenerate, &c->evFinal, &c->evFork, &c->evJoin,
+                          &c->evSummed};
     for (cudaEvent_t* e : evs)
         if (*e)
             cudaEventDestroy(*e);
@@ -993,7 +996,8 @@ tr_status tr_adjoint_frame(void* ctx, void* stream, const float* pixel_grad, flo
     // the replay keeps the forward frame's statistics: its queues are reused, its counters are its own
     FrameView f = c->frame;
     f.counters = c->adjointCounters;
-    TR_CUDA(c, launch_adjoint(c->scene, f, c->camera, c->settings, a, c->shape, pick_stream(c, stream)));
+    TR_CUDA(c, launch_adjoint(c->scene, f, c->camera, c->settings, a, c->shape,
+                              AdjointStreams{c->side, c->evFork, c->evJoin, c->evSummed}, pick_stream(c, stream)));
     return TR_OK;
 }
 

@@ -1816,7 +1816,7 @@ __global__ void __launch_bounds__(256) adjoint_generate_kernel(FrameView f, Came
 // takes this vertex's emission off the remaining radiance): the radiance
 // still unaccounted for arrived through that direction.
 template <bool SMEM>
-__global__ void __launch_bounds__(kAdjointThreads) ext_grad_kernel(SceneView s, FrameView f, uint32_t bounce,
+__global__ void __launch_bounds__(kAdjointThreads, 7) ext_grad_kernel(SceneView s, FrameView f, uint32_t bounce,
                                                                    AdjointView a)
 {
     extern __shared__ float sgrad[];
@@ -1860,7 +1860,7 @@ __global__ void __launch_bounds__(kAdjointThreads) ext_grad_kernel(SceneView s, 
 // extend ray (with its direction kept as the path's pending record) like the
 // forward shade.
 template <bool SMEM>
-__global__ void __launch_bounds__(kAdjointThreads, 4) adjoint_shade_kernel(SceneView s, FrameView f, Settings st,
+__global__ void __launch_bounds__(kAdjointThreads, 5) adjoint_shade_kernel(SceneView s, FrameView f, Settings st,
                                                                         uint32_t bounce, AdjointView a)
 {
     extern __shared__ float sgrad[];
@@ -2026,7 +2026,7 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) adjoint_connect_kernel(SceneV
 // Gradients of the visible NEE contributions: d log f of the light direction
 // at the vertex, and the light's emission.
 template <bool SMEM>
-__global__ void __launch_bounds__(kAdjointThreads) nee_grad_kernel(SceneView s, FrameView f, uint32_t bounce,
+__global__ void __launch_bounds__(kAdjointThreads, 7) nee_grad_kernel(SceneView s, FrameView f, uint32_t bounce,
                                                                    AdjointView a)
 {
     extern __shared__ float sgrad[];
@@ -2259,8 +2259,26 @@ cudaError_t launch_finalize(const FrameView& f, const Settings& st, cudaStream_t
     return cudaGetLastError();
 }
 
+namespace {
+// Resident blocks per SM of `kernel` at `threads` per block (4 when the query fails).
+template <class Kernel>
+uint32_t resident(Kernel kernel, uint32_t threads, size_t smem)
+{
+    int perSm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, int(threads), smem);
+    return uint32_t(perSm > 0 ? perSm : 4);
+}
+} // namespace
+
+// Per bounce: extend, the gradients of the previous vertex's extend direction, shade; then the
+// vertex's visibility and its light gradients, which share no queue with the next bounce's
+// extend launch and run beside it on par.side. The remaining radiance that connect updates is
+// read by the next extend gradients (wait for `connected`), the shadow queue and its payload
+// are rewritten by the next shade (wait for `summed`). In sequence the late bounces of an open
+// scene each waited for the slowest ray of four launches.
 cudaError_t launch_adjoint(const SceneView& s0, const FrameView& f, const Camera& cam, const Settings& st,
-                           const AdjointView& a, const LaunchShape& shape, cudaStream_t stream)
+                           const AdjointView& a, const LaunchShape& shape, const AdjointStreams& par,
+                           cudaStream_t stream)
 {
     const SceneView s = traced(s0, st);
     if (f.pathCount == 0)
@@ -2268,59 +2286,53 @@ cudaError_t launch_adjoint(const SceneView& s0, const FrameView& f, const Camera
     cudaError_t e = cudaMemsetAsync(f.counters, 0, kCounterWords * sizeof(uint32_t), stream);
     if (e != cudaSuccess)
         return e;
-    const size_t smem = size_t(kAdjointWarps) * a.materialCount * kGradSlots * sizeof(float);
-    const bool useSmem = smem <= kAdjointSmemMax;
-    int perSm = 0;
-    e = useSmem ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, adjoint_shade_kernel<true>, kAdjointThreads,
-                                                                smem)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, adjoint_shade_kernel<false>, kAdjointThreads,
-                                                                0);
-    if (e != cudaSuccess)
-        return e;
-    const uint32_t gradBlocks = shape.sms * uint32_t(perSm > 0 ? perSm : 1);
+    const size_t table = size_t(kAdjointWarps) * a.materialCount * kGradSlots * sizeof(float);
+    const bool useSmem = table <= kAdjointSmemMax;
+    const size_t smem = useSmem ? table : 0;
+    const auto shade = useSmem ? adjoint_shade_kernel<true> : adjoint_shade_kernel<false>;
+    const auto extGrad = useSmem ? ext_grad_kernel<true> : ext_grad_kernel<false>;
+    const auto neeGrad = useSmem ? nee_grad_kernel<true> : nee_grad_kernel<false>;
+    const auto connect = s.tlasNodes ? (s.quantNodes ? adjoint_connect_kernel<true, kLayoutQuant>
+                                                     : adjoint_connect_kernel<true, kLayoutWide>)
+                                     : (s.quantNodes ? adjoint_connect_kernel<false, kLayoutQuant>
+                                                     : adjoint_connect_kernel<false, kLayoutWide>);
+    const auto extend = s.tlasNodes ? (s.quantNodes ? extend_kernel<false, false, false, true, kLayoutQuant>
+                                                    : extend_kernel<false, false, false, true, kLayoutWide>)
+                                    : (s.quantNodes ? extend_kernel<false, false, false, false, kLayoutQuant>
+                                                    : extend_kernel<false, false, false, false, kLayoutWide>);
+    const uint32_t shadeBlocks = shape.sms * resident(shade, kAdjointThreads, smem);
+    const uint32_t extBlocks = shape.sms * resident(extGrad, kAdjointThreads, smem);
+    const uint32_t neeBlocks = shape.sms * resident(neeGrad, kAdjointThreads, smem);
     // the replay's connect runs 128-thread blocks: as many threads as the forward connect grid
     const uint32_t connectBlocks128 = (shape.connectBlocks * shape.traversalThreads + 127u) / 128u;
     Settings fwd = st;
     fwd.flags &= ~uint32_t(TR_FLAG_COUNT_TRAVERSAL | TR_FLAG_WRITE_AOVS);
     fwd.refillBelow = shape.refillBelow;
     adjoint_generate_kernel<<<(f.pathCount + 255u) / 256u, 256, 0, stream>>>(f, cam, fwd, a);
-    for (uint32_t bounce = 0; bounce < st.maxDepth; ++bounce) {
-        if (s.tlasNodes && !s.quantNodes)
-            extend_kernel<false, false, false, true, kLayoutWide>
-                <<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, fwd, bounce, Camera{});
-        else if (s.tlasNodes)
-            extend_kernel<false, false, false, true, kLayoutQuant>
-                <<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, fwd, bounce, Camera{});
-        else if (s.quantNodes)
-            extend_kernel<false, false, false, false, kLayoutQuant>
-                <<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, fwd, bounce, Camera{});
-        else
-            extend_kernel<false, false, false, false, kLayoutWide>
-                <<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, fwd, bounce, Camera{});
+    for (uint32_t bounce = 0; e == cudaSuccess && bounce < st.maxDepth; ++bounce) {
+        extend<<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, fwd, bounce, Camera{});
         if (bounce > 0) {
-            if (useSmem)
-                ext_grad_kernel<true><<<gradBlocks, kAdjointThreads, smem, stream>>>(s, f, bounce, a);
-            else
-                ext_grad_kernel<false><<<gradBlocks, kAdjointThreads, 0, stream>>>(s, f, bounce, a);
+            e = cudaStreamWaitEvent(stream, par.connected, 0);
+            extGrad<<<extBlocks, kAdjointThreads, smem, stream>>>(s, f, bounce, a);
+            if (e == cudaSuccess)
+                e = cudaStreamWaitEvent(stream, par.summed, 0);
         }
-        if (useSmem)
-            adjoint_shade_kernel<true><<<gradBlocks, kAdjointThreads, smem, stream>>>(s, f, fwd, bounce, a);
-        else
-            adjoint_shade_kernel<false><<<gradBlocks, kAdjointThreads, 0, stream>>>(s, f, fwd, bounce, a);
-        if (s.tlasNodes && !s.quantNodes)
-            adjoint_connect_kernel<true, kLayoutWide><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
-        else if (s.tlasNodes)
-            adjoint_connect_kernel<true, kLayoutQuant><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
-        else if (s.quantNodes)
-            adjoint_connect_kernel<false, kLayoutQuant><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
-        else
-            adjoint_connect_kernel<false, kLayoutWide><<<connectBlocks128, 128, 0, stream>>>(s, f, fwd, bounce, a);
-        if (useSmem)
-            nee_grad_kernel<true><<<gradBlocks, kAdjointThreads, smem, stream>>>(s, f, bounce, a);
-        else
-            nee_grad_kernel<false><<<gradBlocks, kAdjointThreads, 0, stream>>>(s, f, bounce, a);
+        shade<<<shadeBlocks, kAdjointThreads, smem, stream>>>(s, f, fwd, bounce, a);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(par.shaded, stream);
+        if (e == cudaSuccess)
+            e = cudaStreamWaitEvent(par.side, par.shaded, 0);
+        connect<<<connectBlocks128, 128, 0, par.side>>>(s, f, fwd, bounce, a);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(par.connected, par.side);
+        neeGrad<<<neeBlocks, kAdjointThreads, smem, par.side>>>(s, f, bounce, a);
+        if (e == cudaSuccess)
+            e = cudaEventRecord(par.summed, par.side);
     }
-    return cudaGetLastError();
+    if (e == cudaSuccess)
+        e = cudaStreamWaitEvent(stream, par.summed, 0);
+    const cudaError_t launched = cudaGetLastError();
+    return e != cudaSuccess ? e : launched;
 }
 
 cudaError_t launch_debug_bounce(const SceneView& s0, const FrameView& f, const Camera& cam, const Settings& st,
@@ -2366,15 +2378,6 @@ cudaError_t launch_batch_finalize(const FrameView& f, uint32_t pixelBegin, uint3
 }
 
 namespace {
-// Resident blocks per SM of `kernel` at `threads` per block (4 when the query fails).
-template <class Kernel>
-uint32_t resident(Kernel kernel, uint32_t threads, size_t smem)
-{
-    int perSm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, int(threads), smem);
-    return uint32_t(perSm > 0 ? perSm : 4);
-}
-
 // Block sizes the traversal and shade kernels take: their register budgets are
 // set for blocks of at most 128 threads.
 bool valid_threads(uint32_t t) { return t == 64u || t == 128u; }

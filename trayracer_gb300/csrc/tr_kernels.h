@@ -64,7 +64,14 @@ cudaError_t launch_batch_finalize(const FrameView& f, uint32_t pixelBegin, uint3
 // Path-replay adjoint of the frame `f` (its per-path radiance and sample
 // count are the forward frame's; its queues are overwritten, its counters
 // are the adjoint's own).
+// The streams and events of launch_adjoint: a bounce's visibility and light gradients run on
+// `side` beside the next bounce's extend launch.
+struct AdjointStreams {
+    cudaStream_t side;
+    cudaEvent_t shaded, connected, summed;
+};
 cudaError_t launch_adjoint(const SceneView& s, const FrameView& f, const Camera& cam, const Settings& st,
-                           const AdjointView& a, const LaunchShape& shape, cudaStream_t stream);
+                           const AdjointView& a, const LaunchShape& shape, const AdjointStreams& par,
+                           cudaStream_t stream);
 
 } // namespace tr
