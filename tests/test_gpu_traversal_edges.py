@@ -37,3 +37,44 @@ def test_frames_match_the_oracle(name, w, h, ms, layout):
             close = (np.abs(img[..., :3] - ref) <= 1e-4 * np.maximum(1.0, np.abs(ref))).all(axis=-1)
             # a last-bit difference may flip a sampling decision of a path: one pixel in a hundred
             assert (~close).sum() <= max(1, 0.01 * close.size), (close.mean(), graph)
+
+
+@pytest.mark.parametrize("name,w,h,ms,depth,rr,ref", [
+    ("cornell", 3, 1, 1, 5, 1 << 30, False),      # taken at bounce 3 with fewer paths than a warp
+    ("cornell", 64, 48, 1, 16, 1, False),
+    ("lambert", 61, 37, 2, 16, 1, True),          # the reference's sampling
+    ("disney", 256, 256, 2, 9, 1 << 30, False),   # too many at bounce 3, still too many at 6
+    ("cornell", 300, 200, 3, 12, 2, False),       # too many at bounce 3, taken at 6
+    ("sky", 160, 90, 2, 8, 3, False),             # paths that leave
+    ("textured", 50, 41, 1, 8, 2, False),
+    ("instanced", 50, 41, 1, 8, 2, False),
+])
+def test_captured_frames_equal_eager_ones(name, w, h, ms, depth, rr, ref):
+    """A captured frame hands its remaining paths to one launch where a late bounce holds few
+    (from bounce 3 or 6 of frames of 5 bounces and more): the eager frames' ray counts, and their
+    images to the rounding of separately compiled shading code."""
+    scene = {"cornell": lambda: tr.cornell_box(width=w, height=h),
+             "lambert": lambda: tr.cornell_box(width=w, height=h, wall_closure=tr.TR_CLOSURE_LAMBERT),
+             "disney": lambda: tr.cornell_box(width=w, height=h, wall_closure=tr.TR_CLOSURE_DISNEY),
+             "sky": lambda: tr.outdoor_heightfield(n=64, width=w, height=h),
+             "textured": lambda: tr.textured_cornell(width=w, height=h),
+             "instanced": lambda: tr.instanced_cornell(width=w, height=h)}[name]()
+    st = tr.KernelSettings(multiSample=ms, maxDepth=depth, rrStart=rr, seed=9,
+                           flags=tr.TR_FLAG_REFERENCE_SAMPLING if ref else 0)
+    with tr.DeviceRenderer(0) as r:
+        r.UpdateScene(scene)
+        r.SetCamera(scene.camera)
+        r.Resize((w, h))
+        if name == "sky":
+            r.SetSky(tr.SkySettings(sunDir=(0.2, 0.6, 0.4)))
+        r.SetSettings(st)
+        got = []
+        for graph in (False, True):
+            r.Reset()
+            for _ in range(3):
+                r.RenderFrame(use_graph=graph)
+            s = r.Statistics()
+            got.append((r.ColorBuffer().copy(), s["extend_rays"], s["shadow_rays"], s["hit_rays"], s["device_error"]))
+    assert got[0][1:] == got[1][1:] and got[0][4] == 0
+    # 3 frames of a few products each differ by at most some ulps of the 10.0 radiance limit
+    assert np.abs(got[0][0] - got[1][0]).max() <= 1e-5

@@ -422,6 +422,46 @@ tr_status enqueue_begin(Context* c, cudaStream_t s)
     return TR_OK;
 }
 
+// Extend, shade and connect of bounces [first, last) of a path-traced frame.
+tr_status enqueue_bounces(Context* c, cudaStream_t s, uint32_t first, uint32_t last, bool timed)
+{
+    // default sampling mode: the camera rays are made inside the first extend launch
+    const bool fused = (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING) == 0;
+    // Untimed (captured) frames overlap bounce b's connect with bounce b + 1's
+    // extend: connect reads the shadow queue and adds to the radiance of paths
+    // in flight, extend reads the extend queue and writes the hit queue, so they
+    // share nothing; shade b + 1 (which rewrites the shadow queue and adds
+    // emission to the same radiance) waits for both. Not with a sky: extend
+    // adds the sky to the radiance of missed paths. Timed frames keep the
+    // stages in sequence for their per-stage events.
+    const bool overlap = !timed && !c->scene.sky.enabled;
+    for (uint32_t b = first; b < last; ++b) {
+        TR_CUDA(c, launch_extend(c->scene, c->frame, c->settings, b, c->shape, s, fused ? &c->camera : nullptr));
+        if (c->shape.sortHits)
+            TR_CUDA(c, launch_sort_hits(c->scene, c->frame, c->sort, b, c->shape, s));
+        if (timed)
+            TR_CUDA(c, cudaEventRecord(c->evExtend[b], s));
+        if (overlap && b > first)
+            TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
+        TR_CUDA(c, launch_shade(c->scene, c->frame, c->settings, b, c->shape, s));
+        if (timed)
+            TR_CUDA(c, cudaEventRecord(c->evShade[b], s));
+        if (overlap) {
+            TR_CUDA(c, cudaEventRecord(c->evFork, s));
+            TR_CUDA(c, cudaStreamWaitEvent(c->side, c->evFork, 0));
+            TR_CUDA(c, launch_connect(c->scene, c->frame, c->settings, b, c->shape, c->side));
+            TR_CUDA(c, cudaEventRecord(c->evJoin, c->side));
+        } else {
+            TR_CUDA(c, launch_connect(c->scene, c->frame, c->settings, b, c->shape, s));
+        }
+        if (timed)
+            TR_CUDA(c, cudaEventRecord(c->evConnect[b], s));
+    }
+    if (overlap && last > first)
+        TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
+    return TR_OK;
+}
+
 tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
 {
     tr_status st = enqueue_begin(c, s);
@@ -457,41 +497,80 @@ tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
         TR_CUDA(c, launch_generate(c->frame, c->camera, c->settings, s));
     if (timed)
         TR_CUDA(c, cudaEventRecord(c->evGenerate, s));
-    // Untimed (captured) frames overlap bounce b's connect with bounce b + 1's
-    // extend: connect reads the shadow queue and adds to the radiance of paths
-    // in flight, extend reads the extend queue and writes the hit queue, so they
-    // share nothing; shade b + 1 (which rewrites the shadow queue and adds
-    // emission to the same radiance) waits for both. Not with a sky: extend
-    // adds the sky to the radiance of missed paths. Timed frames keep the
-    // stages in sequence for their per-stage events.
-    const bool overlap = !timed && !c->scene.sky.enabled;
-    for (uint32_t b = 0; b < c->settings.maxDepth; ++b) {
-        TR_CUDA(c, launch_extend(c->scene, c->frame, c->settings, b, c->shape, s, fused ? &c->camera : nullptr));
-        if (c->shape.sortHits)
-            TR_CUDA(c, launch_sort_hits(c->scene, c->frame, c->sort, b, c->shape, s));
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evExtend[b], s));
-        if (overlap && b > 0)
-            TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
-        TR_CUDA(c, launch_shade(c->scene, c->frame, c->settings, b, c->shape, s));
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evShade[b], s));
-        if (overlap) {
-            TR_CUDA(c, cudaEventRecord(c->evFork, s));
-            TR_CUDA(c, cudaStreamWaitEvent(c->side, c->evFork, 0));
-            TR_CUDA(c, launch_connect(c->scene, c->frame, c->settings, b, c->shape, c->side));
-            TR_CUDA(c, cudaEventRecord(c->evJoin, c->side));
-        } else {
-            TR_CUDA(c, launch_connect(c->scene, c->frame, c->settings, b, c->shape, s));
-        }
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evConnect[b], s));
-    }
-    if (overlap)
-        TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
+    const tr_status bst = enqueue_bounces(c, s, 0, c->settings.maxDepth, timed);
+    if (bst != TR_OK)
+        return bst;
     TR_CUDA(c, launch_finalize(c->frame, c->settings, s));
     if (timed)
         TR_CUDA(c, cudaEventRecord(c->evFinal, s));
+    return TR_OK;
+}
+
+// Bounces of a captured frame from which one launch may take the remaining paths (tail_kernel);
+// each is worth its launch when at least two bounces follow.
+constexpr uint32_t kTailBounces[] = {3, 6};
+
+// A path-traced frame as a graph: its bounces, with a tail_kernel launch before the bounces of
+// kTailBounces and the launches between them behind its condition.
+tr_status capture_frame(Context* c, cudaGraph_t g)
+{
+    cudaStream_t s = c->stream;
+    const uint32_t depth = c->settings.maxDepth;
+    tr_status st = TR_OK;
+    auto check = [&](cudaError_t e, const char* what) { st = e == cudaSuccess ? TR_OK : cuda_fail(c, e, what); };
+    cudaGraphNode_t last = nullptr;
+    cudaGraphConditionalHandle handle{};  // whether the bounces after the last tail launch are still to run
+    for (uint32_t from = 0, to = 0; to < depth; from = to) {
+        to = depth;
+        for (uint32_t b : kTailBounces)
+            if (b > from && b + 2u <= depth && b < to)
+                to = b;
+        cudaGraphConditionalHandle next{};
+        if (to < depth)
+            TR_CUDA(c, cudaGraphConditionalHandleCreate(&next, g, 0u, cudaGraphCondAssignDefault));
+        if (from > 0) {
+            cudaGraphNodeParams cp{};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = handle;
+            cp.conditional.type = cudaGraphCondTypeIf;
+            cp.conditional.size = 1;
+            cudaGraphNode_t node = nullptr;
+            TR_CUDA(c, cudaGraphAddNode(&node, g, &last, nullptr, 1, &cp));
+            last = node;
+            const cudaError_t e = capture_into(
+                s, cp.conditional.phGraph_out[0], nullptr, 0,
+                [&]() {
+                    st = enqueue_bounces(c, s, from, to, false);
+                    return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
+                },
+                nullptr);
+            if (st != TR_OK)
+                return st;
+            TR_CUDA(c, e);
+        }
+        // (one kernel ends each capture: the next node's only dependency)
+        const cudaError_t e = capture_into(
+            s, g, last ? &last : nullptr, last ? 1 : 0,
+            [&]() {
+                if (from == 0) {
+                    st = enqueue_begin(c, s);
+                    if (st == TR_OK && (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING))
+                        check(launch_generate(c->frame, c->camera, c->settings, s), "launch_generate");
+                    if (st == TR_OK)
+                        st = enqueue_bounces(c, s, 0, to, false);
+                }
+                if (st == TR_OK && to < depth)
+                    check(launch_tail(c->scene, c->frame, c->settings, to, c->shape, next, s), "launch_tail");
+                else if (st == TR_OK)
+                    check(launch_finalize(c->frame, c->settings, s), "launch_finalize");
+                return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
+            },
+            &last);
+        if (st != TR_OK)
+            return st;
+        TR_CUDA(c, e);
+        handle = next;
+    }
     return TR_OK;
 }
 
@@ -1437,10 +1516,19 @@ tr_status tr_render_frame(void* ctx, void* stream, int32_t use_graph)
     if (use_graph) {
         if (!c->graphValid) {
             // capture on the context stream (the legacy default stream cannot be captured)
-            TR_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            st = enqueue_frame(c, c->stream, false);
             cudaGraph_t g = nullptr;
-            const cudaError_t ec = cudaStreamEndCapture(c->stream, &g);
+            cudaError_t ec;
+            const bool tails = c->renderMode == kModePathTracing && c->settings.maxDepth >= kTailBounces[0] + 2u &&
+                               (c->settings.flags & TR_FLAG_COUNT_TRAVERSAL) == 0;
+            if (tails) {
+                TR_CUDA(c, cudaGraphCreate(&g, 0));
+                st = capture_frame(c, g);
+                ec = cudaSuccess;
+            } else {
+                TR_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+                st = enqueue_frame(c, c->stream, false);
+                ec = cudaStreamEndCapture(c->stream, &g);
+            }
             if (st != TR_OK) {
                 if (g)
                     cudaGraphDestroy(g);

@@ -72,4 +72,29 @@ cudaError_t capture_continuous(const ContinuousLaunch& L, const std::vector<Cont
 cudaError_t run_continuous_eager(const ContinuousLaunch& L, const std::vector<ContinuousRound>& rounds,
                                  uint32_t advance, cudaStream_t s, StageTimes* times = nullptr);
 
+// Captures body() on s into `into` after `deps`; *tail (optional) gets the
+// last node captured.
+template <class Body>
+cudaError_t capture_into(cudaStream_t s, cudaGraph_t into, const cudaGraphNode_t* deps, size_t nDeps, Body&& body,
+                         cudaGraphNode_t* tail)
+{
+    cudaError_t e = cudaStreamBeginCaptureToGraph(s, into, deps, nullptr, nDeps, cudaStreamCaptureModeThreadLocal);
+    if (e != cudaSuccess)
+        return e;
+    e = body();
+    if (e == cudaSuccess && tail) {
+        cudaStreamCaptureStatus cs;
+        const cudaGraphNode_t* d = nullptr;
+        size_t n = 0;
+        e = cudaStreamGetCaptureInfo(s, &cs, nullptr, nullptr, &d, nullptr, &n);
+        if (e == cudaSuccess)
+            *tail = n ? d[n - 1] : nullptr;
+        if (e == cudaSuccess && !*tail)
+            e = cudaErrorStreamCaptureInvalidated;
+    }
+    cudaGraph_t out = into;
+    const cudaError_t ee = cudaStreamEndCapture(s, &out);
+    return e != cudaSuccess ? e : ee;
+}
+
 } // namespace tr

@@ -303,6 +303,9 @@ constexpr uint32_t kConnectWorkBase = 3 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kHitCounterBase = 4 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kVisibleCounterBase = 5 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kCounterWords = 6 * (TR_MAX_DEPTH + 1);
+// (a word of the connect cursors that no bounce uses) set to the bounce from which tail_kernel has
+// taken a frame's remaining paths
+constexpr uint32_t kTailTaken = kConnectWorkBase + TR_MAX_DEPTH;
 
 // Path index / flag packing, Tracer/Common/CommonStructs.h:46-71.
 constexpr uint32_t kPathIxShift = 4;

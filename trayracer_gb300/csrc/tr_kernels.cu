@@ -22,6 +22,7 @@
 #include "tr_kernels.h"
 #include "tr_sky.h"
 
+#include <algorithm>
 #include <type_traits>
 
 #include "tr_bsdf.cuh"
@@ -1333,6 +1334,110 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, F
     }
 }
 
+// A frame's last paths, each followed to its end by one thread. From some bounce on a frame
+// holds a few thousand rays, and every further bounce costs three launches that last as long as
+// their slowest ray: 333 us for a 256 x 256, 1 spp frame of 16 bounces alone on the GPU, two
+// thirds of it after the third bounce. If the bounce's extend queue holds at most kTailPaths
+// rays, this kernel does what the remaining extend, shade and connect launches would (the same
+// traversal and shading, the counters and each path's radiance in the same order), without
+// queues; else it only sets the condition under which the frame's graph goes on with them. A
+// warp takes as few paths as fill the grid: their divergent loops then hardly wait for one another.
+constexpr uint32_t kTailPaths = 32768;
+
+__device__ __noinline__ bool tail_closest(const SceneView& s, float3 O, float3 D, float tmin, float& tmax,
+                                          uint32_t& slot, float& u, float& v, uint32_t& inst)
+{
+    return traverse<false>(s, O, D, tmin, tmax, slot, u, v, nullptr, &inst);
+}
+__device__ __noinline__ bool tail_any(const SceneView& s, float3 O, float3 D, float tmin, float tmax, bool& occluded)
+{
+    uint32_t slot = 0xffffffffu;
+    float u = 0.f, v = 0.f;
+    const bool ok = traverse<true>(s, O, D, tmin, tmax, slot, u, v);
+    occluded = slot != 0xffffffffu;
+    return ok;
+}
+
+template <bool REF, bool TEX>
+__global__ void __launch_bounds__(128) tail_kernel(const __grid_constant__ SceneView s,
+                                                   const __grid_constant__ FrameView f,
+                                                   const __grid_constant__ Settings st, uint32_t bounce,
+                                                   cudaGraphConditionalHandle rest)
+{
+    using Rng = std::conditional_t<REF, RefRng, CounterRng>;
+    // (set to its bounce by the launch that takes the paths: blocks of it that start late see theirs)
+    const uint32_t taken = __ldcg(f.counters + kTailTaken);
+    const uint32_t count = taken != 0u && taken != bounce ? 0u : __ldcg(f.counters + bounce);
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        cudaGraphSetConditional(rest, count > kTailPaths ? 1u : 0u);
+    if (count == 0u || count > kTailPaths)
+        return;
+    // queue lengths of the bounces walked here: extend, hit and shadow rays
+    __shared__ uint32_t tally[3][TR_MAX_DEPTH + 1];
+    for (uint32_t i = threadIdx.x; i < 3u * (TR_MAX_DEPTH + 1u); i += blockDim.x)
+        tally[i / (TR_MAX_DEPTH + 1u)][i % (TR_MAX_DEPTH + 1u)] = 0u;
+    __syncthreads();
+    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t each = (count + warps - 1u) / warps;  // at most 32: the grid has kTailPaths / 32 warps or more
+    const uint32_t i = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * each + lane_id();
+    if (lane_id() < each && i < count) {
+        const uint32_t cap = f.capacity;
+        const uint32_t wh = f.resX * f.resY;
+        const uint32_t sc = *f.sampleCount;
+        float4 O4 = __ldcs(f.state[0] + i), D4 = __ldcs(f.state[0] + i + cap), T4 = __ldcs(f.state[0] + i + 2 * cap);
+        for (uint32_t b = bounce; b < st.maxDepth; ++b) {
+            float tmax = kDstMax, u = 0.f, v = 0.f;
+            uint32_t slot = 0xffffffffu, inst = 0;
+            if (!tail_closest(s, f3(O4), f3(D4), st.rayEpsilon, tmax, slot, u, v, inst))
+                atomicOr(f.errorFlag, 1u);
+            if (slot == 0xffffffffu) {
+                if (s.sky.enabled)
+                    sky_miss<false>(s, f, st, b, O4, D4, T4, false);
+                break;
+            }
+            atomicAdd(&tally[1][b], 1u);
+            const uint4 hd = make_uint4(encode_bary(u, v), inst, __float_as_uint(__ldg(s.bvhTris + 3u * slot).w),
+                                        __float_as_uint(tmax));
+            const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
+            Rng rng;
+            if constexpr (REF)
+                rng = RefRng{tea2(st.seed + pathIx, sc + b + 1u)};
+            else
+                rng.init(pathIx % wh, sc + pathIx / wh, b + 1u, st.seed);
+            bool wantExt = false, wantShadow = false;
+            float4 ext[3], sh[3];
+            shade_path<REF, Rng, TEX>(s, f, st, b, sc, O4, D4, T4, hd, rng, wantExt, ext, wantShadow, sh);
+            if (wantShadow) {
+                atomicAdd(&tally[2][b], 1u);
+                bool occluded;
+                if (!tail_any(s, f3(sh[0]), f3(sh[1]), st.rayEpsilon, sh[1].w - (2 * st.rayEpsilon), occluded))
+                    atomicOr(f.errorFlag, 1u);
+                if (!occluded) {
+                    const float4 r = f.radiance[pathIx];
+                    f.radiance[pathIx] = make_float4(r.x + sh[2].x, r.y + sh[2].y, r.z + sh[2].z, r.w);
+                }
+            }
+            if (!wantExt)
+                break;
+            atomicAdd(&tally[0][b + 1u], 1u);
+            O4 = ext[0];
+            D4 = ext[1];
+            T4 = ext[2];
+        }
+    }
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k <= TR_MAX_DEPTH; k += blockDim.x) {
+        if (tally[0][k])
+            atomicAdd(f.counters + k, tally[0][k]);
+        if (tally[1][k])
+            atomicAdd(f.counters + kHitCounterBase + k, tally[1][k]);
+        if (tally[2][k])
+            atomicAdd(f.counters + kShadowCounterBase + k, tally[2][k]);
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0)
+        f.counters[kTailTaken] = bounce;
+}
+
 // Sums each pixel's samples in sample order into the accumulator and writes
 // colors = accumulator / sampleCount (FinalizeFrame; the film initialisation
 // of optix.cu:181-188 happens here: a frame with sampleCount == 0 overwrites).
@@ -2238,6 +2343,19 @@ cudaError_t launch_connect(const SceneView& s0, const FrameView& f, const Settin
         twoLevel(std::false_type{});
     else
         oneLevel(std::false_type{});
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tail(const SceneView& s0, const FrameView& f, const Settings& st, uint32_t bounce,
+                        const LaunchShape& shape, cudaGraphConditionalHandle rest, cudaStream_t stream)
+{
+    const SceneView s = traced(s0, st);
+    const bool ref = (st.flags & TR_FLAG_REFERENCE_SAMPLING) != 0;
+    const auto kernel = s.texSlots ? (ref ? tail_kernel<true, true> : tail_kernel<false, true>)
+                                   : (ref ? tail_kernel<true, false> : tail_kernel<false, false>);
+    // a warp for every path up to four blocks per SM
+    const uint32_t blocks = std::max((std::min(f.pathCount, kTailPaths) + 127u) / 128u, shape.sms * 4u);
+    kernel<<<blocks, 128, 0, stream>>>(s, f, st, bounce, rest);
     return cudaGetLastError();
 }
 
