@@ -99,6 +99,7 @@ struct Context {
     // host copies kept for material updates without a BVH rebuild
     std::vector<LightTri> hostLights;
     std::vector<uint32_t> hostMatIdx;
+    std::vector<uint32_t> hostMatTris;   // triangles of each material
     uint32_t materialCount = 0;
 
     // settings / camera
@@ -935,6 +936,9 @@ tr_status tr_scene_upload(void* ctx, const tr_scene_desc* desc)
         in.scene_bounds[i] = fs.bounds[i];
     c->hostLights = fs.lights;
     c->hostMatIdx = fs.matIdx;
+    c->hostMatTris.assign(desc->material_count, 0u);
+    for (uint32_t m : fs.matIdx)
+        ++c->hostMatTris[m];
     c->geom.assign(*desc);
     c->meshTriBase = fs.meshTriBase;
     c->leafSize = opt.maxLeafSize;
@@ -961,10 +965,10 @@ tr_status tr_update_materials(void* ctx, const tr_material_desc* materials, uint
             return fail(c, TR_ERR_INVALID_ARGUMENT, "unknown closure");
     // the emissive triangles must stay the same set: only their radiance may change
     size_t emissiveTris = 0;
-    for (uint32_t m : c->hostMatIdx) {
+    for (uint32_t m = 0; m < count; ++m) {
         const tr_material_desc& d = materials[m];
         if (d.emissive[0] + d.emissive[1] + d.emissive[2] > kEpsilon)
-            ++emissiveTris;
+            emissiveTris += c->hostMatTris[m];
     }
     if (emissiveTris != c->hostLights.size())
         return fail(c, TR_ERR_INVALID_ARGUMENT, "the set of emissive triangles changed: upload the scene again");
@@ -1013,10 +1017,14 @@ tr_status tr_update_materials(void* ctx, const tr_material_desc* materials, uint
                               cudaMemcpyHostToDevice));
     }
     c->hostLights = lights;
-    c->scene.lightEnergy = lights.empty() ? 0.f : lights.back().sumEnergy;
+    // light energies are kernel parameters of the captured frames; everything else that changed
+    // is read from the buffers they point at
+    const float lightEnergy = lights.empty() ? 0.f : lights.back().sumEnergy;
+    if (lightEnergy != c->scene.lightEnergy || sumEnergy != c->scene.lightEnergyTotal)
+        invalidate_graph(c);
+    c->scene.lightEnergy = lightEnergy;
     c->scene.lightEnergyTotal = sumEnergy;
     c->info.light_energy = sumEnergy;
-    invalidate_graph(c);  // light energies are kernel parameters
     return tr_reset(ctx);
 }
 
