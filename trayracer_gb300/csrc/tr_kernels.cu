@@ -203,7 +203,8 @@ __device__ __forceinline__ void camera_ray(const Camera& cam, uint32_t resX, uin
     const float aspect = rx / ry;
     float2 screen = make_float2((((float(ix) + jx) / rx) * 2.0f) - 1.f, (((float(iy) + jy) / ry) * 2.0f) - 1.f);
     screen.y /= aspect;
-    const float2 ccd = sample_bokeh(cam, rng, rtl) * cam.aperture;
+    // a pinhole's lens point is its centre whatever is drawn (nothing draws from rng after it)
+    const float2 ccd = cam.aperture != 0.f ? sample_bokeh(cam, rng, rtl) * cam.aperture : make_float2(0.f, 0.f);
     float2 lens = make_float2((cam.tanFov2 * screen.x) - (ccd.x / cam.focalDist),
                               (cam.tanFov2 * screen.y) - (ccd.y / cam.focalDist));
     if (!distort(lens, cam.tanFov2, cam.distortion))
@@ -1468,35 +1469,71 @@ __global__ void __launch_bounds__(256) finalize_kernel(FrameView f, Settings st)
 
 // Closest hit of every ray of the bounce's queue (state[bounce & 1]); the
 // wireframe mode re-aims secondary rays at a jittered point of the pixel as
-// the Secondary raygen program does (optix.cu:292-300).
-__global__ void __launch_bounds__(128) debug_extend_kernel(SceneView s, FrameView f, Camera cam, Settings st,
-                                                           uint32_t bounce)
+// the Secondary raygen program does (optix.cu:292-300). Persistent warps with
+// lane refill as extend_kernel (a thread a ray left a warp waiting for its
+// longest ray: 720p occlusion image of a heightfield 347 -> 340 us, alone on the
+// GPU 583 -> 501 us).
+template <bool TL, int LAYOUT>
+__global__ void __launch_bounds__(128, 8) debug_extend_kernel(SceneView s, FrameView f, Camera cam, Settings st,
+                                                              uint32_t bounce)
 {
     const uint32_t count = queue_length(f, bounce);
-    float4* q = f.state[bounce & 1u];
+    const float4* __restrict__ q = f.state[bounce & 1u];
     const uint32_t cap = f.capacity;
-    const uint32_t sc = *f.sampleCount;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float4 O4 = q[i];
-        float3 O = f3(O4), D = f3(q[i + cap]);
-        const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
-        if (st.renderMode == kModeWireframe && bounce > 0) {
-            const uint32_t wh = f.resX * f.resY;
-            const uint32_t pixelIx = pathIx % wh;
-            RefRng rng{tea2(st.seed + pathIx, (sc << 1) | 1u)};
-            float T;
-            camera_ray(cam, f.resX, f.resY, pixelIx % f.resX, pixelIx / f.resX, rng,
-                       (st.flags & TR_FLAG_REFERENCE_DRAW_RTL) != 0, O, D, T);
+    uint32_t* work = f.counters + kExtendWorkBase + bounce;
+    const uint32_t lane = lane_id();
+    __shared__ uint32_t rayIx[kTraversalThreadsMax];  // queue entry of this thread's ray
+    typename TravOf<TL>::type t;
+    uint2 stack[kTraversalStack];
+    bool alive = false, ended = false, more = true;
+    while (true) {
+        const uint32_t idle = more ? __ballot_sync(kFull, !alive) : 0u;
+        const uint32_t leader = idle ? __ffs(idle) - 1u : 0u;
+        uint32_t first = 0;
+        if (idle && lane == leader)
+            first = atomicAdd(work, __popc(idle));
+        if (ended) {
+            if (!base(t).ok)
+                atomicOr(f.errorFlag, 1u);
+            const uint32_t slot = base(t).hitSlot;
+            f.hits[rayIx[threadIdx.x]] =
+                slot != 0xffffffffu ? make_uint4(encode_bary(base(t).u, base(t).v), hit_instance(t),
+                                                 __float_as_uint(__ldg(s.bvhTris + 3u * slot).w),
+                                                 __float_as_uint(base(t).tmax))
+                                    : make_uint4(0u, 0xffffffffu, 0xffffffffu, __float_as_uint(kDstMax));
+            ended = false;
         }
-        float tmax = kDstMax;
-        uint32_t slot = 0xffffffffu, inst = 0;
-        float u = 0.f, v = 0.f;
-        if (!traverse<false>(s, O, D, st.rayEpsilon, tmax, slot, u, v, nullptr, &inst))
-            atomicOr(f.errorFlag, 1u);
-        f.hits[i] = slot != 0xffffffffu
-                        ? make_uint4(encode_bary(u, v), inst, __float_as_uint(__ldg(s.bvhTris + 3u * slot).w),
-                                     __float_as_uint(tmax))
-                        : make_uint4(0u, 0xffffffffu, 0xffffffffu, __float_as_uint(kDstMax));
+        if (idle) {
+            first = __shfl_sync(kFull, first, leader);
+            const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
+            if (!alive && i < count) {
+                const float4 O4 = q[i];
+                float3 O = f3(O4), D = f3(q[i + cap]);
+                if (st.renderMode == kModeWireframe && bounce > 0) {
+                    const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
+                    const uint32_t pixelIx = pathIx % (f.resX * f.resY);
+                    RefRng rng{tea2(st.seed + pathIx, (*f.sampleCount << 1) | 1u)};
+                    float T;
+                    camera_ray(cam, f.resX, f.resY, pixelIx % f.resX, pixelIx / f.resX, rng,
+                               (st.flags & TR_FLAG_REFERENCE_DRAW_RTL) != 0, O, D, T);
+                }
+                rayIx[threadIdx.x] = i;
+                traversal_begin<LAYOUT>(t, O, D, kDstMax);
+                alive = true;
+            }
+            more = first + __popc(idle) < count;
+        }
+        if (!__any_sync(kFull, alive))
+            break;
+        const uint32_t below = more ? st.refillBelow : 1u;
+        uint32_t active;
+        do {
+            if (alive && traversal_step<false, false, LAYOUT>(t, st.rayEpsilon, stack, s, nullptr)) {
+                alive = false;
+                ended = true;
+            }
+            active = __ballot_sync(kFull, alive);
+        } while (uint32_t(__popc(active)) >= below);
     }
 }
 
@@ -2458,7 +2495,13 @@ cudaError_t launch_debug_bounce(const SceneView& s0, const FrameView& f, const C
 {
     const SceneView s = traced(s0, st);
     const uint32_t blocks = shape.sms * 8u;
-    debug_extend_kernel<<<blocks, 128, 0, stream>>>(s, f, cam, st, bounce);
+    const auto extend = s.tlasNodes ? (s.quantNodes ? debug_extend_kernel<true, kLayoutQuant>
+                                                    : debug_extend_kernel<true, kLayoutWide>)
+                                    : (s.quantNodes ? debug_extend_kernel<false, kLayoutQuant>
+                                                    : debug_extend_kernel<false, kLayoutWide>);
+    Settings traced_st = st;
+    traced_st.refillBelow = shape.refillBelow;
+    extend<<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, cam, traced_st, bounce);
     debug_shade_kernel<<<blocks, 128, 0, stream>>>(s, f, cam, st, bounce);
     return cudaGetLastError();
 }
