@@ -49,10 +49,10 @@ def test_frames_match_the_oracle(name, w, h, ms, layout):
     ("textured", 50, 41, 1, 8, 2, False),
     ("instanced", 50, 41, 1, 8, 2, False),
 ])
-def test_captured_frames_equal_eager_ones(name, w, h, ms, depth, rr, ref):
-    """A captured frame hands its remaining paths to one launch where a late bounce holds few
-    (from bounce 3 or 6 of frames of 5 bounces and more): the eager frames' ray counts, and their
-    images to the rounding of separately compiled shading code."""
+def test_frames_equal_their_stages(name, w, h, ms, depth, rr, ref):
+    """A frame hands its remaining paths to one launch where a late bounce holds few (from bounce
+    3 or 6 of frames of 5 bounces and more): the ray counts of the stage entries, which launch
+    every bounce, and their images to the rounding of separately compiled shading code."""
     scene = {"cornell": lambda: tr.cornell_box(width=w, height=h),
              "lambert": lambda: tr.cornell_box(width=w, height=h, wall_closure=tr.TR_CLOSURE_LAMBERT),
              "disney": lambda: tr.cornell_box(width=w, height=h, wall_closure=tr.TR_CLOSURE_DISNEY),
@@ -69,12 +69,22 @@ def test_captured_frames_equal_eager_ones(name, w, h, ms, depth, rr, ref):
             r.SetSky(tr.SkySettings(sunDir=(0.2, 0.6, 0.4)))
         r.SetSettings(st)
         got = []
-        for graph in (False, True):
+        for how in ("stages", "eager", "graph"):
             r.Reset()
             for _ in range(3):
-                r.RenderFrame(use_graph=graph)
+                if how != "stages":
+                    r.RenderFrame(use_graph=how == "graph")
+                    continue
+                r.BeginFrame()
+                r.Generate()
+                for b in range(depth):
+                    r.Extend(b)
+                    r.Shade(b)
+                    r.Connect(b)
+                r.Finalize()
             s = r.Statistics()
             got.append((r.ColorBuffer().copy(), s["extend_rays"], s["shadow_rays"], s["hit_rays"], s["device_error"]))
-    assert got[0][1:] == got[1][1:] and got[0][4] == 0
-    # 3 frames of a few products each differ by at most some ulps of the 10.0 radiance limit
-    assert np.abs(got[0][0] - got[1][0]).max() <= 1e-5
+    for g in got[1:]:
+        assert got[0][1:] == g[1:] and g[4] == 0
+        # 3 frames of a few products each differ by at most some ulps of the 10.0 radiance limit
+        assert np.abs(got[0][0] - g[0]).max() <= 1e-5
