@@ -532,9 +532,11 @@ __device__ __noinline__ void sky_miss(const SceneView& s, const FrameView& f, co
 // paths carried over from the last iteration, the entries after them start
 // new samples (their camera rays are made here), so the pool stays full.
 // Blocks of 64 or 128 threads (a launch parameter, LaunchShape::traversalThreads):
-// the kernel works per warp; 64 registers, 32 resident warps per SM.
+// the kernel works per warp; 64 registers, 32 resident warps per SM (two levels, whose
+// traversal holds more: 72 registers and 7 blocks, two-level frame 2529 us against 2594 at 8
+// blocks, 2552 at 6 and 2670 at 5).
 template <bool COUNT, bool BATCH, bool PRIMARY, bool TL, int LAYOUT>
-__global__ void __launch_bounds__(128, 8) extend_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
+__global__ void __launch_bounds__(128, TL ? 7 : 8) extend_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
                                                      Camera cam)
 {
     const uint32_t count = BATCH ? __ldcg(&f.batch->queue) : queue_length(f, bounce);
