@@ -88,3 +88,26 @@ def test_frames_equal_their_stages(name, w, h, ms, depth, rr, ref):
         assert got[0][1:] == g[1:] and g[4] == 0
         # 3 frames of a few products each differ by at most some ulps of the 10.0 radiance limit
         assert np.abs(got[0][0] - g[0]).max() <= 1e-5
+
+
+@pytest.mark.parametrize("ref,mode", [(False, tr.RenderModes.PathTracing), (True, tr.RenderModes.PathTracing),
+                                      (False, tr.RenderModes.AmbientOcclusion)])
+def test_stage_times_of_an_eager_frame(ref, mode):
+    """Stage times are differences of the launches' start times: none negative, together within
+    the frame's time between its events (5 us for the timers' steps)."""
+    scene = tr.cornell_box(width=128, height=96)
+    with tr.DeviceRenderer(0) as r:
+        r.UpdateScene(scene)
+        r.SetCamera(scene.camera)
+        r.Resize((128, 96))
+        st = tr.KernelSettings(multiSample=2, maxDepth=16, rrStart=1,
+                               flags=tr.TR_FLAG_REFERENCE_SAMPLING if ref else 0)
+        for _ in range(3):
+            r.RenderFrame(st, mode)
+        s = r.Statistics()
+        stages = [s[f"{k}_time_ms"] for k in ("generate", "extend", "shade", "connect", "finalize")]
+        assert min(stages) >= 0.0 and stages[1] > 0.0 and stages[4] > 0.0
+        assert sum(stages) <= s["render_time_ms"] + 0.005
+        if mode == tr.RenderModes.PathTracing:
+            assert stages[2] > 0.0 and stages[3] > 0.0
+            assert sum(stages) >= 0.5 * s["render_time_ms"]

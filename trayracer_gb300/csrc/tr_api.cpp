@@ -119,6 +119,7 @@ struct Context {
     uint32_t frameW = 0, frameH = 0, frameMs = 0;
     LaunchShape shape{};
     uint32_t sampleCount = 0;
+    unsigned long long* stamps = nullptr;  // kStamps words of the frame arena (eager frames' stage times)
     float* pickResult = nullptr;       // 9 words of the frame arena (tr_pick_ray)
     float* pickHost = nullptr;         // 9 words of mapped host memory, where there is some
 
@@ -129,14 +130,14 @@ struct Context {
     std::vector<TexSlots> texSlotsHost;
 
     // timing
-    cudaEvent_t evStart = nullptr, evGenerate = nullptr, evFinal = nullptr;
+    cudaEvent_t evStart = nullptr, evFinal = nullptr;
     // captured frames trace bounce b's shadow rays on this stream while bounce
     // b + 1's extend rays run on the frame's stream (fork / join)
     cudaStream_t side = nullptr;
     cudaEvent_t evFork = nullptr, evJoin = nullptr;
     cudaEvent_t evSummed = nullptr;    // tr_adjoint_frame: a bounce's light gradients are summed
-    cudaEvent_t evExtend[TR_MAX_DEPTH] = {}, evShade[TR_MAX_DEPTH] = {}, evConnect[TR_MAX_DEPTH] = {};
     bool timedFrame = false;
+    bool timedGenerate = false, timedStages = false;  // it had a generate launch; path tracing's stages
     uint32_t timedDepth = 0;
     cudaStream_t lastStream = nullptr;
 
@@ -370,6 +371,7 @@ tr_status ensure_frame(Context* c)
     const size_t oKeys = take(cap * sizeof(uint32_t));
     const size_t oOrder = take(cap * sizeof(uint32_t));
     const size_t oPick = take(16 * sizeof(float));
+    const size_t oStamps = take(kStamps * sizeof(unsigned long long));
     void* base = nullptr;
     const cudaError_t e = cudaMalloc(&base, off);
     if (e != cudaSuccess)
@@ -394,6 +396,7 @@ tr_status ensure_frame(Context* c)
     c->sort.keys = reinterpret_cast<uint32_t*>(b + oKeys);
     c->sort.order = reinterpret_cast<uint32_t*>(b + oOrder);
     c->pickResult = reinterpret_cast<float*>(b + oPick);
+    c->stamps = reinterpret_cast<unsigned long long*>(b + oStamps);
     f.capacity = uint32_t(cap);
     f.resX = c->width;
     f.resY = c->height;
@@ -441,13 +444,9 @@ tr_status enqueue_bounces(Context* c, cudaStream_t s, uint32_t first, uint32_t l
         TR_CUDA(c, launch_extend(c->scene, c->frame, c->settings, b, c->shape, s, fused ? &c->camera : nullptr));
         if (c->shape.sortHits)
             TR_CUDA(c, launch_sort_hits(c->scene, c->frame, c->sort, b, c->shape, s));
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evExtend[b], s));
         if (overlap && b > first)
             TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
         TR_CUDA(c, launch_shade(c->scene, c->frame, c->settings, b, c->shape, s));
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evShade[b], s));
         if (overlap) {
             TR_CUDA(c, cudaEventRecord(c->evFork, s));
             TR_CUDA(c, cudaStreamWaitEvent(c->side, c->evFork, 0));
@@ -456,8 +455,6 @@ tr_status enqueue_bounces(Context* c, cudaStream_t s, uint32_t first, uint32_t l
         } else {
             TR_CUDA(c, launch_connect(c->scene, c->frame, c->settings, b, c->shape, s));
         }
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evConnect[b], s));
     }
     if (overlap && last > first)
         TR_CUDA(c, cudaStreamWaitEvent(s, c->evJoin, 0));
@@ -478,15 +475,8 @@ tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
         st.aoDist = c->aoDist;
         st.zDepthMax = c->zDepthMax;
         TR_CUDA(c, launch_generate(c->frame, c->camera, st, s));
-        if (timed)
-            TR_CUDA(c, cudaEventRecord(c->evGenerate, s));
         for (uint32_t b = 0; b < st.maxDepth; ++b) {
             TR_CUDA(c, launch_debug_bounce(c->scene, c->frame, c->camera, st, b, c->shape, s));
-            if (timed) {
-                TR_CUDA(c, cudaEventRecord(c->evExtend[b], s));
-                TR_CUDA(c, cudaEventRecord(c->evShade[b], s));
-                TR_CUDA(c, cudaEventRecord(c->evConnect[b], s));
-            }
         }
         TR_CUDA(c, launch_finalize(c->frame, c->settings, s));
         if (timed)
@@ -497,8 +487,6 @@ tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
     const bool fused = (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING) == 0;
     if (!fused)
         TR_CUDA(c, launch_generate(c->frame, c->camera, c->settings, s));
-    if (timed)
-        TR_CUDA(c, cudaEventRecord(c->evGenerate, s));
     const tr_status bst = enqueue_bounces(c, s, 0, c->settings.maxDepth, timed);
     if (bst != TR_OK)
         return bst;
@@ -768,11 +756,7 @@ tr_status tr_create(const tr_config* config, void** out_ctx)
     ok = ok && cudaEventCreateWithFlags(&c->evFork, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&c->evSummed, cudaEventDisableTiming) == cudaSuccess;
-    ok = ok && cudaEventCreate(&c->evStart) == cudaSuccess && cudaEventCreate(&c->evGenerate) == cudaSuccess &&
-         cudaEventCreate(&c->evFinal) == cudaSuccess;
-    for (uint32_t i = 0; ok && i < TR_MAX_DEPTH; ++i)
-        ok = cudaEventCreate(&c->evExtend[i]) == cudaSuccess && cudaEventCreate(&c->evShade[i]) == cudaSuccess &&
-             cudaEventCreate(&c->evConnect[i]) == cudaSuccess;
+    ok = ok && cudaEventCreate(&c->evStart) == cudaSuccess && cudaEventCreate(&c->evFinal) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         tr_destroy(c);
@@ -799,16 +783,11 @@ tr_status tr_destroy(void* ctx)
     release_textures(c);
     if (c->pickHost)
         cudaFreeHost(c->pickHost);
-    cudaEvent_t* evs[] = {&c->evStart, &c->evGenerate, &c->evFinal, &c->evFork, &c->evJoin,
+    cudaEvent_t* evs[] = {&c->evStart, &c->evFinal, &c->evFork, &c->evJoin,
                           &c->evSummed};
     for (cudaEvent_t* e : evs)
         if (*e)
             cudaEventDestroy(*e);
-    for (uint32_t i = 0; i < TR_MAX_DEPTH; ++i) {
-        if (c->evExtend[i]) cudaEventDestroy(c->evExtend[i]);
-        if (c->evShade[i]) cudaEventDestroy(c->evShade[i]);
-        if (c->evConnect[i]) cudaEventDestroy(c->evConnect[i]);
-    }
     if (c->side)
         cudaStreamDestroy(c->side);
     if (c->stream)
@@ -1569,9 +1548,13 @@ tr_status tr_render_frame(void* ctx, void* stream, int32_t use_graph)
         TR_CUDA(c, cudaGraphLaunch(c->graphExec, s));
         c->timedFrame = false;
     } else {
+        c->frame.stamps = c->stamps;
         st = enqueue_frame(c, s, true);
+        c->frame.stamps = nullptr;
         if (st != TR_OK)
             return st;
+        c->timedStages = c->renderMode == kModePathTracing;
+        c->timedGenerate = !c->timedStages || (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING) != 0;
         c->timedFrame = true;
         c->timedDepth = c->settings.maxDepth;
     }
@@ -1778,20 +1761,23 @@ tr_status tr_get_statistics(void* ctx, tr_statistics* out)
         float ms = 0.f;
         cudaEventElapsedTime(&ms, c->evStart, c->evFinal);
         s.render_time_ms = ms;
-        cudaEventElapsedTime(&ms, c->evStart, c->evGenerate);
-        s.generate_time_ms = ms;
-        cudaEvent_t prev = c->evGenerate;
+        // a stage lasts from its launch to the next one's
+        unsigned long long stamp[kStamps];
+        TR_CUDA(c, cudaMemcpy(stamp, c->stamps, sizeof(stamp), cudaMemcpyDeviceToHost));
+        auto between = [&](uint32_t from, uint32_t to) { return float(double(int64_t(stamp[to] - stamp[from])) * 1e-6); };
+        if (c->timedGenerate)
+            s.generate_time_ms = between(kStampGenerate, kStampExtend);
         for (uint32_t b = 0; b < c->timedDepth; ++b) {
-            cudaEventElapsedTime(&ms, prev, c->evExtend[b]);
-            s.extend_time_ms += ms;
-            cudaEventElapsedTime(&ms, c->evExtend[b], c->evShade[b]);
-            s.shade_time_ms += ms;
-            cudaEventElapsedTime(&ms, c->evShade[b], c->evConnect[b]);
-            s.connect_time_ms += ms;
-            prev = c->evConnect[b];
+            const uint32_t next = b + 1u < c->timedDepth ? kStampExtend + b + 1u : kStampFinalize;
+            if (c->timedStages) {
+                s.extend_time_ms += between(kStampExtend + b, kStampShade + b);
+                s.shade_time_ms += between(kStampShade + b, kStampConnect + b);
+                s.connect_time_ms += between(kStampConnect + b, next);
+            } else {
+                s.extend_time_ms += between(kStampExtend + b, next);  // the other modes' bounces
+            }
         }
-        cudaEventElapsedTime(&ms, prev, c->evFinal);
-        s.finalize_time_ms = ms;
+        s.finalize_time_ms = between(kStampFinalize, kStampEnd);
     }
     s.sample_count = sc;
     s.device_error = err;

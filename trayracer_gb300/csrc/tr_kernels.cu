@@ -52,6 +52,27 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
+// Keeps the device time at which a launch of an eager frame starts.
+__device__ __forceinline__ void stamp(const FrameView& f, uint32_t i)
+{
+    if (f.stamps && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        f.stamps[i] = t;
+    }
+}
+
+// Keeps the device time at which the last warp of a launch ends: connect's start, kept by
+// shade (a stamp of its own made connect_kernel spill 40 bytes more, a sky frame 2 % slower).
+__device__ __forceinline__ void stamp_end(const FrameView& f, uint32_t i)
+{
+    if (f.stamps && lane_id() == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+        atomicMax(f.stamps + i, t);
+    }
+}
+
 // Appends the lanes with pred set to a queue; one atomic per warp.
 __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool pred)
 {
@@ -351,6 +372,7 @@ __device__ __forceinline__ uint32_t camera_order(const FrameView& f, uint32_t i)
 template <bool REF, bool BATCH>
 __global__ void __launch_bounds__(256) generate_kernel(FrameView f, Camera cam, Settings st)
 {
+    stamp(f, kStampGenerate);
     const uint32_t pathIx = blockIdx.x * blockDim.x + threadIdx.x;
     if (pathIx >= f.pathCount)
         return;
@@ -539,6 +561,8 @@ template <bool COUNT, bool BATCH, bool PRIMARY, bool TL, int LAYOUT>
 __global__ void __launch_bounds__(128, TL ? 7 : 8) extend_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce,
                                                      Camera cam)
 {
+    if (!BATCH)
+        stamp(f, kStampExtend + bounce);
     const uint32_t count = BATCH ? __ldcg(&f.batch->queue) : queue_length(f, bounce);
     const uint32_t carried = BATCH ? __ldcg(&f.batch->carried) : 0u;
     const uint32_t freshBase = BATCH ? __ldcg(&f.batch->freshBase) : 0u;
@@ -1068,6 +1092,8 @@ constexpr uint32_t kShadeStageBytes = 2u * 4u * sizeof(float4);
 template <bool REF, bool BATCH, bool TEX = false>
 __global__ void __launch_bounds__(128, 5) shade_kernel(SceneView s, FrameView f, Settings st, uint32_t bounce)
 {
+    if (!BATCH)
+        stamp(f, kStampShade + bounce);
     const uint32_t count = BATCH ? __ldcg(&f.batch->hits) : __ldcg(f.counters + kHitCounterBase + bounce);
     const float4* __restrict__ in = f.state[1];
     float4* __restrict__ out = f.state[0];
@@ -1153,6 +1179,8 @@ __global__ void __launch_bounds__(128, 5) shade_kernel(SceneView s, FrameView f,
             __stcs(out + exSlot + 2 * cap, ext[2]);
         }
     }
+    if (!BATCH)
+        stamp_end(f, kStampConnect + bounce);
 }
 
 // Material sort of the hit queue (optional, chosen by the tuner): a counting
@@ -1446,6 +1474,7 @@ __global__ void __launch_bounds__(128) tail_kernel(const __grid_constant__ Scene
 // of optix.cu:181-188 happens here: a frame with sampleCount == 0 overwrites).
 __global__ void __launch_bounds__(256) finalize_kernel(FrameView f, Settings st)
 {
+    stamp(f, kStampFinalize);
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t wh = f.resX * f.resY;
     if (p >= wh)
@@ -1479,6 +1508,7 @@ template <bool TL, int LAYOUT>
 __global__ void __launch_bounds__(128, 8) debug_extend_kernel(SceneView s, FrameView f, Camera cam, Settings st,
                                                               uint32_t bounce)
 {
+    stamp(f, kStampExtend + bounce);
     const uint32_t count = queue_length(f, bounce);
     const float4* __restrict__ q = f.state[bounce & 1u];
     const uint32_t cap = f.capacity;
@@ -2218,6 +2248,7 @@ __global__ void __launch_bounds__(kAdjointThreads, 7) nee_grad_kernel(SceneView 
 
 __global__ void advance_kernel(FrameView f, Settings st)
 {
+    stamp(f, kStampEnd);
     if (threadIdx.x == 0 && blockIdx.x == 0)
         *f.sampleCount += st.multiSample;
 }
