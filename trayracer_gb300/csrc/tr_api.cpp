@@ -438,7 +438,7 @@ tr_status enqueue_bounces(Context* c, cudaStream_t s, uint32_t first, uint32_t l
     // share nothing; shade b + 1 (which rewrites the shadow queue and adds
     // emission to the same radiance) waits for both. Not with a sky: extend
     // adds the sky to the radiance of missed paths. Timed frames keep the
-    // stages in sequence for their per-stage events.
+    // stages in sequence for their stage times.
     const bool overlap = !timed && !c->scene.sky.enabled;
     for (uint32_t b = first; b < last; ++b) {
         TR_CUDA(c, launch_extend(c->scene, c->frame, c->settings, b, c->shape, s, fused ? &c->camera : nullptr));
