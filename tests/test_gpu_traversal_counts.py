@@ -1,0 +1,105 @@
+"""The traversal kernels on given rays (written into the queues that the stage entries read)
+against the host's run of the same traversal: hits bit for bit, and the nodes and triangles that
+TR_FLAG_COUNT_TRAVERSAL sums up."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import trayracer_gb300 as tr
+from trayracer_gb300 import _abi
+from trayracer_gb300.renderer import SceneDescHolder
+from trayracer_gb300.scenes import random_soup
+
+from test_box_test import CLOSE_CALLS
+
+pytestmark = pytest.mark.gpu
+
+BOUNCES = 17  # counters per bounce: extend and shadow queue lengths, two cursors, hit queue length
+N = 6000      # rays: more than a warp's refill takes, not a multiple of a warp
+
+
+def host_trace(scene, O, D, tmin, any_hit, quant):
+    h = SceneDescHolder(scene)
+    hits = np.zeros((O.shape[0], 4), np.uint32)
+    counts = np.zeros((O.shape[0], 2), np.uint32)
+    st = _abi.load_library().tr_trace_host(C.byref(h.desc), O.ctypes.data, D.ctypes.data, O.shape[0], tmin,
+                                           any_hit | (2 if quant else 0), hits.ctypes.data, counts.ctypes.data)
+    assert st == 0
+    return hits, counts.astype(np.uint64).sum(0)
+
+
+def the_scene(name):
+    if name == "heightfield":
+        return tr.heightfield(n=33, seed=1)
+    if name == "instanced":
+        return tr.instanced_cornell()
+    scene = random_soup(3000, seed=5)
+    if name == "triangle":
+        scene = random_soup(1, seed=2)
+        scene.positions[:] = np.array([[-1, 0, -1], [1, 0, -1], [0, 0, 1]], np.float32)
+    return scene
+
+
+def the_rays(name, scene, seed):
+    rng = np.random.default_rng(seed)
+    O = np.zeros((N, 4), np.float32)
+    D = np.zeros((N, 4), np.float32)
+    O[:, :3] = rng.uniform(-1.0, 1.0, (N, 3)) * (0.8 if name == "instanced" else 1.0)
+    if name == "heightfield":
+        O[:, :3] = scene.camera.position
+    d = rng.normal(size=(N, 3))
+    if name == "heightfield":
+        d[:, 1] = -np.abs(d[:, 1])
+    d[rng.random(N) < 0.1, 1] = 0.0  # along a coordinate plane
+    D[:, :3] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    D[:, 3] = rng.uniform(0.5, 20.0, N)
+    if name == "heightfield":
+        close = np.array([c[1] for c in CLOSE_CALLS], np.uint32).view(np.float32)
+        D[:500, :3] = close[np.arange(500) % len(close)]
+    if name == "triangle":  # from the triangle itself, up and down
+        O[:, :3] = 0.0
+        D[:, :3] = 0.0
+        D[::2, 1], D[1::2, 1] = 1.0, -1.0
+    return O, D
+
+
+def renderer(scene, quant, eps):
+    r = tr.DeviceRenderer(0)
+    r.UpdateScene(scene)
+    r.SetTuning(bvh_nodes=2 if quant else 1)
+    r.SetCamera(scene.camera)
+    r.Resize((N, 1))
+    r.SetSettings(tr.KernelSettings(maxDepth=2, rayEpsilon=eps, flags=_abi.TR_FLAG_COUNT_TRAVERSAL))
+    r.BeginFrame()
+    r.Synchronize()
+    return r, r.Buffers()
+
+
+CASES = [("heightfield", 1e-3), ("soup", 1e-3), ("instanced", 1e-3), ("triangle", 0.0)]
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("name,eps", CASES)
+def test_closest_hits_and_their_counts(name, eps, quant):
+    scene = the_scene(name)
+    O, D = the_rays(name, scene, 3)
+    want, counts = host_trace(scene, O, D, eps, 0, quant)
+    r, buf = renderer(scene, quant, eps)
+    state = np.zeros((3, N, 4), np.float32)
+    state[0], state[1] = O, D
+    state[0][:, 3] = (np.arange(N, dtype=np.uint32) << 4).view(np.float32)
+    r.write_device(buf["path_state"][0], state)
+    r.write_device(buf["counters"] + 4 * 1, np.array([N], np.uint32))  # bounce 1's extend queue
+    r.Extend(1)
+    s = r.Statistics()
+    n_hit = s["hit_rays"][1]
+    path = r.read_device(buf["path_state"][1], np.uint32, n_hit * 4).reshape(n_hit, 4)[:, 3] >> 4
+    hits = r.read_device(buf["hits"], np.uint32, n_hit * 4).reshape(n_hit, 4)
+    r.close()
+    got = np.tile(np.array([0, 0xFFFFFFFF, 0xFFFFFFFF, 0], np.uint32), (N, 1))
+    got[path] = hits
+    hit = want[:, 2] != 0xFFFFFFFF
+    assert s["device_error"] == 0 and n_hit == hit.sum() > 0.05 * N
+    assert (got[hit] == want[hit]).all() and (got[~hit, 2] == 0xFFFFFFFF).all()
+    assert (s["traversal_extend_nodes"], s["traversal_extend_tris"]) == tuple(int(c) for c in counts)
