@@ -250,7 +250,8 @@ typedef struct tr_statistics {
     uint32_t sample_count;          /* accumulated samples per pixel */
     uint32_t device_error;          /* nonzero: a kernel recorded a bounded-loop overrun (traversal stack
                                        depth or traversal_step_limit) since the last tr_reset */
-    /* with TR_FLAG_COUNT_TRAVERSAL, summed over the frames since tr_reset */
+    /* with TR_FLAG_COUNT_TRAVERSAL, summed over the frames since tr_reset: nodes visited and
+       triangles tested, of a shadow ray those up to its first hit */
     uint64_t traversal_extend_nodes;
     uint64_t traversal_extend_tris;
     uint64_t traversal_connect_nodes;

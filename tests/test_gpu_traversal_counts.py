@@ -26,7 +26,7 @@ def host_trace(scene, O, D, tmin, any_hit, quant):
     st = _abi.load_library().tr_trace_host(C.byref(h.desc), O.ctypes.data, D.ctypes.data, O.shape[0], tmin,
                                            any_hit | (2 if quant else 0), hits.ctypes.data, counts.ctypes.data)
     assert st == 0
-    return hits, counts.astype(np.uint64).sum(0)
+    return hits, counts
 
 
 def the_scene(name):
@@ -53,7 +53,7 @@ def the_rays(name, scene, seed):
         d[:, 1] = -np.abs(d[:, 1])
     d[rng.random(N) < 0.1, 1] = 0.0  # along a coordinate plane
     D[:, :3] = d / np.linalg.norm(d, axis=1, keepdims=True)
-    D[:, 3] = rng.uniform(0.5, 20.0, N)
+    D[:, 3] = rng.uniform(0.5, 20.0, N) * (4.0 if name == "heightfield" else 1.0)
     if name == "heightfield":
         close = np.array([c[1] for c in CLOSE_CALLS], np.uint32).view(np.float32)
         D[:500, :3] = close[np.arange(500) % len(close)]
@@ -102,4 +102,43 @@ def test_closest_hits_and_their_counts(name, eps, quant):
     hit = want[:, 2] != 0xFFFFFFFF
     assert s["device_error"] == 0 and n_hit == hit.sum() > 0.05 * N
     assert (got[hit] == want[hit]).all() and (got[~hit, 2] == 0xFFFFFFFF).all()
-    assert (s["traversal_extend_nodes"], s["traversal_extend_tris"]) == tuple(int(c) for c in counts)
+    assert (s["traversal_extend_nodes"], s["traversal_extend_tris"]) == tuple(counts.sum(0, dtype=int))
+
+
+def connect(r, buf, O, D, eps):
+    """Runs bounce 1's connect launch over the given rays (D.w: how far each may be occluded);
+    returns whether each was, and the statistics."""
+    n = O.shape[0]
+    shadow = np.zeros((3, N, 4), np.float32)
+    shadow[0, :n], shadow[1, :n] = O, D
+    shadow[0, :n, 3] = np.arange(n, dtype=np.uint32).view(np.float32)
+    shadow[1, :n, 3] = D[:, 3] + np.float32(2.0) * np.float32(eps)
+    shadow[2, :n, 0] = 1.0
+    r.write_device(buf["shadow"], shadow)
+    r.write_device(buf["radiance"], np.zeros((N, 4), np.float32))
+    r.write_device(buf["counters"] + 4 * (BOUNCES + 1), np.array([n], np.uint32))  # bounce 1's shadow queue
+    r.Connect(1)
+    return r.read_device(buf["radiance"], np.float32, 4 * N).reshape(N, 4)[:n, 0] == 0.0, r.Statistics()
+
+
+def shadow_rays(name, scene, eps, seed):
+    O, D = the_rays(name, scene, seed)
+    # the distance that the kernel is left with after it took 2 eps off again
+    D[:, 3] = (D[:, 3] + np.float32(2.0) * np.float32(eps)) - np.float32(2.0) * np.float32(eps)
+    return O, D
+
+
+@pytest.mark.parametrize("quant", [False, True])
+@pytest.mark.parametrize("name,eps", CASES)
+def test_shadow_rays_and_their_counts(name, eps, quant):
+    """What is visited and tested up to a ray's first hit, although a warp tests the triangles of
+    its rays together."""
+    scene = the_scene(name)
+    O, D = shadow_rays(name, scene, eps, 4)
+    want, counts = host_trace(scene, O, D, eps, 1, quant)
+    r, buf = renderer(scene, quant, eps)
+    occluded, s = connect(r, buf, O, D, eps)
+    r.close()
+    assert s["device_error"] == 0 and 0.05 * N < occluded.sum()
+    assert (occluded == (want[:, 2] != 0xFFFFFFFF)).all()
+    assert (s["traversal_connect_nodes"], s["traversal_connect_tris"]) == tuple(counts.sum(0, dtype=int))

@@ -439,18 +439,24 @@ constexpr uint32_t kTraversalThreadsMax = 128;
 // render (1080p, 64 spp) 91.8 -> 88.4 ms with fp32 nodes, 87.8 -> 83.2 ms with quantized ones.
 // (Closest-hit rays lose with it, 83.2 -> 87.9 ms: what a test finds has to travel back to the
 // owner, and nodes are visited that the hit would cull.)
+template <bool COUNT>
 struct WarpTriangles {
     float4 O[32];      // origin, tmax
     float4 D[32];
     uint2 entry[32];   // triangle slot, owner lane
 };
+template <>
+struct WarpTriangles<true> : WarpTriangles<false> {
+    uint32_t nodes[32];  // nodes that the owner lane had visited when it listed the entry
+};
 // Listed triangles from which the warp tests them at once; fewer wait for more while enough
 // lanes have nodes to visit (16 and 24 within 0.1 %, 8 and 32 1 %, at once 3 % slower).
 constexpr uint32_t kTriangleBatch = 16;
 
-// Tests the listed triangles (count of them); `mine` has a bit for each entry of this lane.
+// Tests the listed triangles (count of them); `mine` has a bit for each entry of this lane. COUNT
+// counts what one ray after the other would have visited and tested: nothing after the first hit.
 template <bool COUNT>
-__device__ __forceinline__ void test_listed(Traversal& t, WarpTriangles& w, float tmin, const SceneView& s,
+__device__ __forceinline__ void test_listed(Traversal& t, WarpTriangles<COUNT>& w, float tmin, const SceneView& s,
                                             uint32_t& count, uint32_t& mine, TraversalCounts* cnt)
 {
     const uint32_t lane = lane_id();
@@ -462,10 +468,17 @@ __device__ __forceinline__ void test_listed(Traversal& t, WarpTriangles& w, floa
         const float4* tp = s.bvhTris + 3u * e.x;
         float tt, uu, vv;
         hit = intersect_triangle(f3(o), f3(d), __ldg(tp + 0), __ldg(tp + 1), __ldg(tp + 2), tmin, o.w, tt, uu, vv);
-        if (COUNT)
-            cnt->tris++;
     }
-    if (__ballot_sync(kFull, hit) & mine)
+    const uint32_t own = __ballot_sync(kFull, hit) & mine;
+    if constexpr (COUNT) {
+        if (t.hitSlot == 0xffffffffu) {
+            // (entries are listed in the order in which a ray finds them)
+            cnt->tris += __popc(own ? mine & (own ^ (own - 1u)) : mine);
+            if (own)
+                cnt->nodes = w.nodes[__ffs(own) - 1u];
+        }
+    }
+    if (own)
         t.hitSlot = 0u;
     mine = 0u;
     count = 0u;
@@ -475,7 +488,7 @@ __device__ __forceinline__ void test_listed(Traversal& t, WarpTriangles& w, floa
 // Visits nodes with the warp's shadow rays until fewer than `below` of them are alive; the rays
 // that end set `ended` (t.hitSlot other than ~0: occluded).
 template <bool COUNT, int LAYOUT>
-__device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles& w, uint2* stack, const SceneView& s,
+__device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles<COUNT>& w, uint2* stack, const SceneView& s,
                                               float tmin, uint32_t below, bool& alive, bool& ended,
                                               TraversalCounts* cnt)
 {
@@ -499,6 +512,8 @@ __device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles& w, ui
             if (tris.y != 0u) {
                 const uint32_t at = count + __popc(m & ((1u << lane) - 1u));
                 w.entry[at] = make_uint2(tris.x + __ffs(tris.y) - 1u, lane);
+                if constexpr (COUNT)
+                    w.nodes[at] = cnt->nodes;
                 mine |= 1u << at;
                 tris.y &= tris.y - 1u;
             }
@@ -514,8 +529,13 @@ __device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles& w, ui
         active = __ballot_sync(kFull, alive);
     } while (uint32_t(__popc(active)) >= below);
     // (rays that ended leave their lanes to others: nothing of theirs stays listed)
-    if (count)
+    if (count) {
         test_listed<COUNT>(t, w, tmin, s, count, mine, cnt);
+        if (COUNT && alive && t.hitSlot != 0xffffffffu) {
+            alive = false;  // (no more nodes to be counted; else its next step ends it)
+            ended = true;
+        }
+    }
 }
 
 // Closest hit of the bounce's extend queue. Rays that hit are appended (one
@@ -1300,7 +1320,7 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, F
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
     __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
-    __shared__ WarpTriangles warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
+    __shared__ WarpTriangles<COUNT> warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
     bool alive = false, ended = false, more = true;
     while (true) {
         // The rays that ended since the last refill, all lanes at once: the contribution of
@@ -2135,7 +2155,7 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) adjoint_connect_kernel(SceneV
     typename TravOf<TL>::type t;
     uint2 stack[kTraversalStack];
     __shared__ uint2 rayIds[kTraversalThreadsMax];  // shadow slot and path of this thread's ray
-    __shared__ WarpTriangles warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
+    __shared__ WarpTriangles<false> warpTris[TL ? 1 : kTraversalThreadsMax / 32u];
     bool alive = false, ended = false, more = true;
     while (true) {
         // the rays that ended since the last refill, all lanes at once (as connect_kernel)
