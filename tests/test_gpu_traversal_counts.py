@@ -64,13 +64,14 @@ def the_rays(name, scene, seed):
     return O, D
 
 
-def renderer(scene, quant, eps):
+def renderer(scene, quant, eps, step_limit=0):
     r = tr.DeviceRenderer(0)
     r.UpdateScene(scene)
     r.SetTuning(bvh_nodes=2 if quant else 1)
     r.SetCamera(scene.camera)
     r.Resize((N, 1))
-    r.SetSettings(tr.KernelSettings(maxDepth=2, rayEpsilon=eps, flags=_abi.TR_FLAG_COUNT_TRAVERSAL))
+    r.SetSettings(tr.KernelSettings(maxDepth=2, rayEpsilon=eps, flags=_abi.TR_FLAG_COUNT_TRAVERSAL,
+                                    traversalStepLimit=step_limit))
     r.BeginFrame()
     r.Synchronize()
     return r, r.Buffers()
@@ -142,3 +143,22 @@ def test_shadow_rays_and_their_counts(name, eps, quant):
     assert s["device_error"] == 0 and 0.05 * N < occluded.sum()
     assert (occluded == (want[:, 2] != 0xFFFFFFFF)).all()
     assert (s["traversal_connect_nodes"], s["traversal_connect_tris"]) == tuple(counts.sum(0, dtype=int))
+
+
+@pytest.mark.parametrize("name", ["heightfield", "soup"])
+def test_a_hit_within_the_step_limit_is_no_error(name):
+    """Occluded rays at the step limit that each reaches its hit with, and one step below it."""
+    scene = the_scene(name)
+    O, D = shadow_rays(name, scene, 1e-3, 6)
+    want, counts = host_trace(scene, O, D, 1e-3, 1, False)
+    hit = want[:, 2] != 0xFFFFFFFF
+    steps = counts[hit, 0]
+    limit = int(np.median(steps))
+    for ok, chosen in ((True, steps <= limit), (False, steps == limit + 1)):
+        o, d = np.ascontiguousarray(O[hit][chosen]), np.ascontiguousarray(D[hit][chosen])
+        assert o.shape[0] > 100
+        r, buf = renderer(scene, False, 1e-3, limit)
+        occluded, s = connect(r, buf, o, d, 1e-3)
+        r.close()
+        assert s["device_error"] == (0 if ok else 1)
+        assert occluded.all() if ok else not occluded.all()

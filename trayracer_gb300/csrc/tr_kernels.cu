@@ -538,6 +538,13 @@ __device__ __forceinline__ void trace_shadows(Traversal& t, WarpTriangles<COUNT>
     }
 }
 
+// Whether a shadow ray that ended passed a bound: not if the triangles that were listed when it ran
+// out of steps held its hit, at which it had ended before.
+__device__ __forceinline__ bool shadow_bound_passed(const Traversal& t, const SceneView& s)
+{
+    return !t.ok && (t.hitSlot == 0xffffffffu || t.steps <= s.stepLimit);
+}
+
 // Closest hit of the bounce's extend queue. Rays that hit are appended (one
 // warp ballot and one atomic per step) to the hit queue with their full path
 // state and hit record; missed rays end here. COUNT = true also sums the nodes
@@ -1331,7 +1338,7 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, F
         if (idle && lane == leader)
             first = atomicAdd(work, __popc(idle));
         if (ended) {
-            if (!base(t).ok)
+            if (shadow_bound_passed(base(t), s))
                 atomicOr(f.errorFlag, 1u);
             if (base(t).hitSlot == 0xffffffffu) {
                 const uint2 ids = rayIds[threadIdx.x];
@@ -2169,7 +2176,7 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) adjoint_connect_kernel(SceneV
             slot = atomicAdd(visCounter, __popc(vis));
         if (idle && lane == leader)
             first = atomicAdd(work, __popc(idle));
-        if (ended && !base(t).ok)
+        if (ended && shadow_bound_passed(base(t), s))
             atomicOr(f.errorFlag, 1u);
         if (vis) {
             slot = __shfl_sync(kFull, slot, visLeader) + __popc(vis & ((1u << lane) - 1u));
