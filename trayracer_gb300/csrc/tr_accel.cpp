@@ -87,7 +87,12 @@ SceneAccel build_accel(const tr_scene_desc& desc, const std::vector<uint32_t>& m
 bool quantize_accel(const SceneAccel& acc, bool wanted, std::vector<QuantNode>& nodes,
                     std::vector<QuantNode>& tlasNodes)
 {
-    return wanted && acc.quantizable && quantize_nodes(acc.nodes, nodes) && quantize_nodes(acc.tlasNodes, tlasNodes);
+    if (!wanted || !acc.quantizable)
+        return false;
+    const std::vector<WideNode>& top = acc.tlasNodes.empty() ? acc.nodes : acc.tlasNodes;
+    if (top.empty() || !(largest_extent(top[0]) >= kQuantMinExtent))
+        return false;
+    return quantize_nodes(acc.nodes, nodes) && quantize_nodes(acc.tlasNodes, tlasNodes);
 }
 
 } // namespace tr

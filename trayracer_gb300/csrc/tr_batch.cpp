@@ -411,7 +411,10 @@ tr_status tr_batch_create(const tr_config* config, const tr_batch_item* items, u
     };
     // the node layout of the concatenated BVHs (one-level scenes: by their node count)
     std::vector<QuantNode> qnodes;
-    const bool quant = quantized_nodes(nodes.size(), 0u) && quantize_nodes(nodes, qnodes);
+    bool quant = quantized_nodes(nodes.size(), 0u);
+    for (const BatchItem& it : b->items)
+        quant = quant && largest_extent(nodes[it.root]) >= kQuantMinExtent;
+    quant = quant && quantize_nodes(nodes, qnodes);
     const void* nodeSrc = quant ? static_cast<const void*>(qnodes.data()) : static_cast<const void*>(nodes.data());
     const size_t nodeBytes = nodes.size() * (quant ? sizeof(QuantNode) : sizeof(WideNode));
     const size_t oNodes = take(nodeBytes);

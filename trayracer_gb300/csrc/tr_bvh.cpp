@@ -617,6 +617,20 @@ Cwbvh collapse_to_cwbvh(const BinaryBvh& bvh, const float* positions, const uint
         t.join();
     return out;
 }
+float largest_extent(const WideNode& root)
+{
+    float most = 0.f;
+    for (int a = 0; a < 3; ++a) {
+        float lo = INFINITY, hi = -INFINITY;  // (empty slots are +inf .. -inf)
+        for (int sl = 0; sl < 8; ++sl) {
+            lo = std::min(lo, root.lo[a][sl]);
+            hi = std::max(hi, root.hi[a][sl]);
+        }
+        most = std::max(most, hi - lo);
+    }
+    return most;
+}
+
 bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& out)
 {
     out.assign(nodes.size(), QuantNode{});

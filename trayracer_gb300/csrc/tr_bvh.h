@@ -69,6 +69,12 @@ Cwbvh collapse_to_cwbvh(const BinaryBvh& bvh, const float* positions, const uint
 // fit a float at the traversal's scale (2^42 * step * 1e20 < 2^127).
 constexpr float kQuantMaxExtent = 0x1p24f;
 bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& out);
+// Smallest extent of a scene's box (along its longest axis) that the quantized layout takes. Its
+// distances are denormal below 2^-26 along the ray, with steps of 2^-49: in a scene of this
+// extent still finer than the rounding of its coordinates' differences.
+constexpr float kQuantMinExtent = 0x1p-33f;
+// The longest axis of the box of a BVH's root node.
+float largest_extent(const WideNode& root);
 // Largest magnification of a ray's direction into an instance's space that the
 // quantized layout takes (its reciprocal, at the traversal's scale, must not be
 // denormal); scenes beyond keep fp32 child boxes.
