@@ -1,7 +1,9 @@
-"""Where the quantized node layout hands over to fp32 child boxes: scenes too small for its scaled
-distances. Host traversal: the layout asked for finds the same hits, hit for hit, at every scale."""
+"""The ends of what the quantized node layout's scaled distances take: scenes too small for them (fp32
+child boxes serve), directions far from unit length. Host traversal, hit for hit."""
 import numpy as np
 import pytest
+
+import trayracer_gb300 as tr
 
 from test_box_test import _trace
 from trayracer_gb300.scenes import random_soup
@@ -31,3 +33,26 @@ def test_small_scenes(exponent, falls_back):
     assert (want[:, 2] != 0xFFFFFFFF).mean() > 0.3
     assert (got == want).all()
     assert (counts == wide).all() == falls_back
+
+
+@pytest.mark.parametrize("any_hit", [0, 1])
+@pytest.mark.parametrize("exponent", [-20, 2, 20, 27, 40])
+@pytest.mark.parametrize("name", ["soup", "instanced"])
+def test_long_and_short_directions(name, exponent, any_hit):
+    """Directions scaled by a power of two: the same hits and visits, distances scaled the other way.
+    The instances magnify directions by 2^18."""
+    scene = random_soup(3000, seed=5)
+    O, D = _rays(5000, 9)
+    if name == "instanced":
+        scene = tr.instanced_cornell()
+        scene.instances = [(m, x * np.float32(2.0**-18)) for m, x in scene.instances]
+        O[:, :3] *= np.float32(0.7 * 2.0**-18)
+    want, counts = _trace(scene, O, D, 0.0, any_hit | 2)
+    scale = np.float32(2.0) ** exponent
+    D[:, :3] *= scale
+    D[:, 3] /= scale
+    got, counts2 = _trace(scene, O, D, 0.0, any_hit | 2)
+    hit = want[:, 2] != 0xFFFFFFFF
+    assert hit.mean() > 0.3
+    assert (got[:, :3] == want[:, :3]).all() and (counts == counts2).all()
+    assert (got[hit, 3].view(np.float32) * scale == want[hit, 3].view(np.float32)).all()

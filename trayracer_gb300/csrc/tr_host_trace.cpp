@@ -5,6 +5,7 @@
 // tested) can be counted.
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <thread>
 #include <vector>
 
@@ -17,7 +18,7 @@
 using namespace tr;
 
 extern "C" tr_status tr_trace_host(const tr_scene_desc* desc, const float* O4, const float* D4, uint32_t n,
-                                   float tmin, int32_t any_hit, uint32_t* hits, uint32_t* counts)
+                                   float rayTmin, int32_t any_hit, uint32_t* hits, uint32_t* counts)
 {
     if (!desc || (n && (!O4 || !D4 || !hits)))
         return TR_ERR_INVALID_ARGUMENT;
@@ -48,8 +49,20 @@ extern "C" tr_status tr_trace_host(const tr_scene_desc* desc, const float* O4, c
     auto work = [&](unsigned t) {
         for (uint32_t i = t; i < n; i += threads) {
             const float3 O = make_float3(O4[4 * i], O4[4 * i + 1], O4[4 * i + 2]);
-            const float3 D = make_float3(D4[4 * i], D4[4 * i + 1], D4[4 * i + 2]);
+            float3 D = make_float3(D4[4 * i], D4[4 * i + 1], D4[4 * i + 2]);
             float tmax = any_hit ? D4[4 * i + 3] : kDstMax;
+            float tmin = rayTmin;
+            // The quantized box test takes directions of about unit length (launches have no
+            // others): a longer one is traced at a power of two of its length, which changes no
+            // rounding, and its distances are scaled with it.
+            int shift = 0;
+            const float longest = fmaxf(fabsf(D.x), fmaxf(fabsf(D.y), fabsf(D.z)));
+            if (quant && longest > 2.0f && std::isfinite(longest)) {
+                std::frexp(longest, &shift);
+                D = make_float3(std::ldexp(D.x, -shift), std::ldexp(D.y, -shift), std::ldexp(D.z, -shift));
+                tmin = std::ldexp(tmin, shift);
+                tmax = std::ldexp(tmax, shift);
+            }
             uint32_t slot = 0xffffffffu;
             float u = 0.f, v = 0.f;
             TraversalCounts c{0, 0};
@@ -65,7 +78,7 @@ extern "C" tr_status tr_trace_host(const tr_scene_desc* desc, const float* O4, c
                 h[0] = (bx << 16) | by;
                 h[1] = inst;
                 h[2] = f2u(acc.tris[3 * size_t(slot)].w);
-                h[3] = f2u(tmax);
+                h[3] = f2u(std::ldexp(tmax, -shift));
             } else {
                 h[0] = 0;
                 h[1] = 0xffffffffu;
