@@ -119,7 +119,7 @@ struct Context {
     uint32_t frameW = 0, frameH = 0, frameMs = 0;
     LaunchShape shape{};
     uint32_t sampleCount = 0;
-    unsigned long long* stamps = nullptr;  // kStamps words of the frame arena (eager frames' stage times)
+    unsigned long long* stamps = nullptr;  // kStamps device words (eager frames' stage times: kept when the frame is resized)
     float* pickResult = nullptr;       // 9 words of the frame arena (tr_pick_ray)
     float* pickHost = nullptr;         // 9 words of mapped host memory, where there is some
 
@@ -371,7 +371,6 @@ tr_status ensure_frame(Context* c)
     const size_t oKeys = take(cap * sizeof(uint32_t));
     const size_t oOrder = take(cap * sizeof(uint32_t));
     const size_t oPick = take(16 * sizeof(float));
-    const size_t oStamps = take(kStamps * sizeof(unsigned long long));
     void* base = nullptr;
     const cudaError_t e = cudaMalloc(&base, off);
     if (e != cudaSuccess)
@@ -396,7 +395,6 @@ tr_status ensure_frame(Context* c)
     c->sort.keys = reinterpret_cast<uint32_t*>(b + oKeys);
     c->sort.order = reinterpret_cast<uint32_t*>(b + oOrder);
     c->pickResult = reinterpret_cast<float*>(b + oPick);
-    c->stamps = reinterpret_cast<unsigned long long*>(b + oStamps);
     f.capacity = uint32_t(cap);
     f.resX = c->width;
     f.resY = c->height;
@@ -757,6 +755,8 @@ tr_status tr_create(const tr_config* config, void** out_ctx)
          cudaEventCreateWithFlags(&c->evJoin, cudaEventDisableTiming) == cudaSuccess &&
          cudaEventCreateWithFlags(&c->evSummed, cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreate(&c->evStart) == cudaSuccess && cudaEventCreate(&c->evFinal) == cudaSuccess;
+    ok = ok && cudaMalloc(reinterpret_cast<void**>(&c->stamps), kStamps * sizeof(unsigned long long)) == cudaSuccess &&
+         cudaMemset(c->stamps, 0, kStamps * sizeof(unsigned long long)) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         tr_destroy(c);
@@ -781,6 +781,8 @@ tr_status tr_destroy(void* ctx)
     c->adjointArena.release();
     c->samplesArena.release();
     release_textures(c);
+    if (c->stamps)
+        cudaFree(c->stamps);
     if (c->pickHost)
         cudaFreeHost(c->pickHost);
     cudaEvent_t* evs[] = {&c->evStart, &c->evFinal, &c->evFork, &c->evJoin,
