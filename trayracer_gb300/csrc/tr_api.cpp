@@ -121,7 +121,8 @@ struct Context {
     uint32_t sampleCount = 0;
     unsigned long long* stamps = nullptr;  // kStamps device words (eager frames' stage times: kept when the frame is resized)
     float* pickResult = nullptr;       // 9 words of the frame arena (tr_pick_ray)
-    float* pickHost = nullptr;         // 9 words of mapped host memory, where there is some
+    float* pickHost = nullptr;         // 9 words of mapped host memory, where there is some,
+    float* pickMapped = nullptr;       // and their device address
 
     // textures of the scene: one CUDA array and texture object each, and the
     // per-material slots as uploaded (kept to rewrite their emissive colour)
@@ -762,6 +763,13 @@ tr_status tr_create(const tr_config* config, void** out_ctx)
         tr_destroy(c);
         return TR_ERR_CUDA;
     }
+    // a pick's answer in mapped host memory; where there is none, picks copy it back
+    if (cudaHostAlloc(reinterpret_cast<void**>(&c->pickHost), 9 * sizeof(float), cudaHostAllocMapped) != cudaSuccess)
+        c->pickHost = nullptr;
+    else if (cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->pickMapped), c->pickHost, 0) != cudaSuccess)
+        c->pickMapped = nullptr;
+    if (!c->pickMapped)
+        cudaGetLastError();
     *out_ctx = c;
     return TR_OK;
 }
@@ -1127,16 +1135,7 @@ tr_status tr_pick_ray(void* ctx, void* stream, int32_t x, int32_t y, tr_ray_pick
     cudaStream_t s = pick_stream(c, stream);
     // the kernel writes its answer where the host reads it (a pick takes 24 us, 32 with a
     // copy back)
-    float* mapped = nullptr;
-    if (!c->pickHost && cudaHostAlloc(reinterpret_cast<void**>(&c->pickHost), 9 * sizeof(float),
-                                      cudaHostAllocMapped) != cudaSuccess) {
-        cudaGetLastError();
-        c->pickHost = nullptr;
-    }
-    if (c->pickHost && cudaHostGetDevicePointer(reinterpret_cast<void**>(&mapped), c->pickHost, 0) != cudaSuccess) {
-        cudaGetLastError();
-        mapped = nullptr;
-    }
+    float* mapped = c->pickMapped;
     TR_CUDA(c, launch_pick_ray(c->scene, c->camera, c->settings, c->width, c->height, x, y,
                                mapped ? mapped : c->pickResult, c->frame.errorFlag, s));
     float r[9];
