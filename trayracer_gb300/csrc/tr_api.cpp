@@ -495,72 +495,99 @@ tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
     return TR_OK;
 }
 
-// Bounces of a captured frame from which one launch may take the remaining paths (tail_kernel);
-// each is worth its launch when at least two bounces follow.
-constexpr uint32_t kTailBounces[] = {3, 6};
+// Where a captured path-traced frame hands its remaining paths to one launch (tail_kernel).
+struct TailPlan {
+    uint32_t bounce = 0;       // 0: nowhere
+    bool conditional = false;  // the launches of the bounces after it stand behind a graph condition
+};
 
-// A path-traced frame as a graph: its bounces, with a tail_kernel launch before the bounces of
-// kTailBounces and the launches between them behind its condition.
-tr_status capture_frame(Context* c, cudaGraph_t g)
+// A frame of at most kTailAlways paths hands them over for sure, and its later launches need not be
+// captured at all (60 x 60, 16 bounces 335 -> 209 us, captured anew each frame 540 -> 269 us). A
+// larger one needs a condition, which costs each capture some 20 us and each frame that keeps its
+// launches 20 us (256 x 256, 5 bounces 141 -> 163 us); it pays where the paths fade: under a sky
+// (960 x 540, 4 spp, 8 bounces 1743 -> 1414 us), or some bounces after Russian roulette sets in with
+// enough bounces to follow (300 x 300, 11 bounces, roulette from 3: 258 -> 191 us). Not in closed
+// rooms without roulette (180 x 180, 16 bounces 369 us, 437 handed over); open scenes without a sky
+// cannot be told from them here. Frames of more paths fade to few some bounces later.
+constexpr uint32_t kTailAlways = 4096;
+TailPlan tail_plan(const Settings& st, uint32_t paths, bool sky)
+{
+    TailPlan plan;
+    uint32_t follow = 0;  // bounces that have to follow
+    if (paths <= kTailAlways) {
+        plan.bounce = 3;
+        follow = 3;
+    } else if (sky) {
+        plan.bounce = paths <= (1u << 22) ? 3u : 4u;
+        plan.conditional = true;
+        follow = 2;
+    } else if (st.rrStart < TR_MAX_DEPTH) {
+        plan.bounce = std::max(3u, st.rrStart + 1u) + (paths > (1u << 17) ? 2u : 0u);
+        plan.conditional = true;
+        follow = 4;
+    }
+    const bool counting = (st.flags & TR_FLAG_COUNT_TRAVERSAL) != 0;  // (tail_kernel keeps no such counts)
+    return plan.bounce && !counting && st.maxDepth >= plan.bounce + follow ? plan : TailPlan{};
+}
+
+// A path-traced frame with a tail_kernel launch as a graph.
+tr_status capture_frame(Context* c, cudaGraph_t g, const TailPlan& plan)
 {
     cudaStream_t s = c->stream;
-    const uint32_t depth = c->settings.maxDepth;
     tr_status st = TR_OK;
     auto check = [&](cudaError_t e, const char* what) { st = e == cudaSuccess ? TR_OK : cuda_fail(c, e, what); };
     cudaGraphNode_t last = nullptr;
-    cudaGraphConditionalHandle handle{};  // whether the bounces after the last tail launch are still to run
-    for (uint32_t from = 0, to = 0; to < depth; from = to) {
-        to = depth;
-        for (uint32_t b : kTailBounces)
-            if (b > from && b + 2u <= depth && b < to)
-                to = b;
-        cudaGraphConditionalHandle next{};
-        if (to < depth)
-            TR_CUDA(c, cudaGraphConditionalHandleCreate(&next, g, 0u, cudaGraphCondAssignDefault));
-        if (from > 0) {
-            cudaGraphNodeParams cp{};
-            cp.type = cudaGraphNodeTypeConditional;
-            cp.conditional.handle = handle;
-            cp.conditional.type = cudaGraphCondTypeIf;
-            cp.conditional.size = 1;
-            cudaGraphNode_t node = nullptr;
-            TR_CUDA(c, cudaGraphAddNode(&node, g, &last, nullptr, 1, &cp));
-            last = node;
-            const cudaError_t e = capture_into(
-                s, cp.conditional.phGraph_out[0], nullptr, 0,
-                [&]() {
-                    st = enqueue_bounces(c, s, from, to, false);
-                    return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
-                },
-                nullptr);
-            if (st != TR_OK)
-                return st;
-            TR_CUDA(c, e);
-        }
-        // (one kernel ends each capture: the next node's only dependency)
+    // captures body() after the last node; one kernel ends each: the next one's only dependency
+    auto capture = [&](auto&& body) -> tr_status {
         const cudaError_t e = capture_into(
             s, g, last ? &last : nullptr, last ? 1 : 0,
             [&]() {
-                if (from == 0) {
-                    st = enqueue_begin(c, s);
-                    if (st == TR_OK && (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING))
-                        check(launch_generate(c->frame, c->camera, c->settings, s), "launch_generate");
-                    if (st == TR_OK)
-                        st = enqueue_bounces(c, s, 0, to, false);
-                }
-                if (st == TR_OK && to < depth)
-                    check(launch_tail(c->scene, c->frame, c->settings, to, c->shape, next, s), "launch_tail");
-                else if (st == TR_OK)
-                    check(launch_finalize(c->frame, c->settings, s), "launch_finalize");
+                body();
                 return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
             },
             &last);
         if (st != TR_OK)
             return st;
         TR_CUDA(c, e);
-        handle = next;
-    }
-    return TR_OK;
+        return TR_OK;
+    };
+    auto finalize = [&]() { check(launch_finalize(c->frame, c->settings, s), "launch_finalize"); };
+    cudaGraphConditionalHandle rest{};  // whether the bounces after the tail launch are still to run
+    if (plan.conditional)
+        TR_CUDA(c, cudaGraphConditionalHandleCreate(&rest, g, 0u, cudaGraphCondAssignDefault));
+    tr_status cs = capture([&]() {
+        st = enqueue_begin(c, s);
+        if (st == TR_OK && (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING))
+            check(launch_generate(c->frame, c->camera, c->settings, s), "launch_generate");
+        if (st == TR_OK)
+            st = enqueue_bounces(c, s, 0, plan.bounce, false);
+        if (st == TR_OK)
+            check(launch_tail(c->scene, c->frame, c->settings, plan.bounce, c->shape,
+                              plan.conditional ? &rest : nullptr, s), "launch_tail");
+        if (st == TR_OK && !plan.conditional)
+            finalize();
+    });
+    if (cs != TR_OK || !plan.conditional)
+        return cs;
+    cudaGraphNodeParams cp{};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = rest;
+    cp.conditional.type = cudaGraphCondTypeIf;
+    cp.conditional.size = 1;
+    cudaGraphNode_t node = nullptr;
+    TR_CUDA(c, cudaGraphAddNode(&node, g, &last, nullptr, 1, &cp));
+    last = node;
+    const cudaError_t e = capture_into(
+        s, cp.conditional.phGraph_out[0], nullptr, 0,
+        [&]() {
+            st = enqueue_bounces(c, s, plan.bounce, c->settings.maxDepth, false);
+            return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
+        },
+        nullptr);
+    if (st != TR_OK)
+        return st;
+    TR_CUDA(c, e);
+    return capture(finalize);
 }
 
 } // namespace
@@ -1524,11 +1551,12 @@ tr_status tr_render_frame(void* ctx, void* stream, int32_t use_graph)
             // capture on the context stream (the legacy default stream cannot be captured)
             cudaGraph_t g = nullptr;
             cudaError_t ec;
-            const bool tails = c->renderMode == kModePathTracing && c->settings.maxDepth >= kTailBounces[0] + 2u &&
-                               (c->settings.flags & TR_FLAG_COUNT_TRAVERSAL) == 0;
-            if (tails) {
+            const TailPlan plan = c->renderMode == kModePathTracing
+                                      ? tail_plan(c->settings, c->frame.pathCount, c->scene.sky.enabled)
+                                      : TailPlan{};
+            if (plan.bounce) {
                 TR_CUDA(c, cudaGraphCreate(&g, 0));
-                st = capture_frame(c, g);
+                st = capture_frame(c, g, plan);
                 ec = cudaSuccess;
             } else {
                 TR_CUDA(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));

@@ -304,8 +304,8 @@ constexpr uint32_t kConnectWorkBase = 3 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kHitCounterBase = 4 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kVisibleCounterBase = 5 * (TR_MAX_DEPTH + 1);
 constexpr uint32_t kCounterWords = 6 * (TR_MAX_DEPTH + 1);
-// (a word of the connect cursors that no bounce uses) set to the bounce from which tail_kernel has
-// taken a frame's remaining paths
+// (a word of the connect cursors that no bounce uses) the bounce from which tail_kernel has taken
+// the frame's remaining paths, 0 if it has not
 constexpr uint32_t kTailTaken = kConnectWorkBase + TR_MAX_DEPTH;
 
 // Launches of an eager frame whose start times are kept (FrameView::stamps, nanoseconds of the

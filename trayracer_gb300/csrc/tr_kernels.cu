@@ -1395,12 +1395,17 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, F
 // A frame's last paths, each followed to its end by one thread. From some bounce on a frame
 // holds a few thousand rays, and every further bounce costs three launches that last as long as
 // their slowest ray: 333 us for a 256 x 256, 1 spp frame of 16 bounces alone on the GPU, two
-// thirds of it after the third bounce. If the bounce's extend queue holds at most kTailPaths
-// rays, this kernel does what the remaining extend, shade and connect launches would (the same
-// traversal and shading, the counters and each path's radiance in the same order), without
-// queues; else it only sets the condition under which the frame's graph goes on with them. A
-// warp takes as few paths as fill the grid: their divergent loops then hardly wait for one another.
+// thirds of it after the third bounce. This kernel does what the remaining extend, shade and
+// connect launches would (the same traversal and shading, the counters and each path's radiance in
+// the same order), without queues; or, if there are too many, it only sets the condition under
+// which the frame's graph goes on with them. A warp takes as few paths as fill the grid: their
+// divergent loops then hardly wait for one another.
+// Too many are more than kTailPaths, and more than kTailPathsSteady where more than two thirds of
+// the last bounce's paths are still there: those go on for many bounces, and a lane whose path ends
+// stays empty (closed room without roulette, 16 bounces: 2500 paths at bounce 3 375 -> 223 us, 6900
+// paths 373 -> 358 us, 22 000 paths 376 -> 440 us; with roulette 20 000 paths 374 -> 290 us).
 constexpr uint32_t kTailPaths = 32768;
+constexpr uint32_t kTailPathsSteady = 4096;
 
 __device__ __noinline__ bool tail_closest(const SceneView& s, float3 O, float3 D, float tmin, float& tmax,
                                           uint32_t& slot, float& u, float& v, uint32_t& inst)
@@ -1420,15 +1425,19 @@ template <bool REF, bool TEX>
 __global__ void __launch_bounds__(128) tail_kernel(const __grid_constant__ SceneView s,
                                                    const __grid_constant__ FrameView f,
                                                    const __grid_constant__ Settings st, uint32_t bounce,
-                                                   cudaGraphConditionalHandle rest)
+                                                   cudaGraphConditionalHandle rest, bool conditional)
 {
     using Rng = std::conditional_t<REF, RefRng, CounterRng>;
-    // (set to its bounce by the launch that takes the paths: blocks of it that start late see theirs)
-    const uint32_t taken = __ldcg(f.counters + kTailTaken);
-    const uint32_t count = taken != 0u && taken != bounce ? 0u : __ldcg(f.counters + bounce);
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        cudaGraphSetConditional(rest, count > kTailPaths ? 1u : 0u);
-    if (count == 0u || count > kTailPaths)
+    const uint32_t count = __ldcg(f.counters + bounce);
+    if (conditional) {
+        const bool steady = 3u * count > 2u * __ldcg(f.counters + bounce - 1u);
+        const bool many = count > (steady ? kTailPathsSteady : kTailPaths);
+        if (blockIdx.x == 0 && threadIdx.x == 0)
+            cudaGraphSetConditional(rest, many ? 1u : 0u);
+        if (many)
+            return;
+    }
+    if (count == 0u)
         return;
     // queue lengths of the bounces walked here: extend, hit and shadow rays
     __shared__ uint32_t tally[3][TR_MAX_DEPTH + 1];
@@ -2444,7 +2453,7 @@ cudaError_t launch_connect(const SceneView& s0, const FrameView& f, const Settin
 }
 
 cudaError_t launch_tail(const SceneView& s0, const FrameView& f, const Settings& st, uint32_t bounce,
-                        const LaunchShape& shape, cudaGraphConditionalHandle rest, cudaStream_t stream)
+                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, cudaStream_t stream)
 {
     const SceneView s = traced(s0, st);
     const bool ref = (st.flags & TR_FLAG_REFERENCE_SAMPLING) != 0;
@@ -2452,7 +2461,7 @@ cudaError_t launch_tail(const SceneView& s0, const FrameView& f, const Settings&
                                    : (ref ? tail_kernel<true, false> : tail_kernel<false, false>);
     // a warp for every path up to four blocks per SM
     const uint32_t blocks = std::max((std::min(f.pathCount, kTailPaths) + 127u) / 128u, shape.sms * 4u);
-    kernel<<<blocks, 128, 0, stream>>>(s, f, st, bounce, rest);
+    kernel<<<blocks, 128, 0, stream>>>(s, f, st, bounce, rest ? *rest : cudaGraphConditionalHandle{}, rest != nullptr);
     return cudaGetLastError();
 }
 

@@ -39,11 +39,11 @@ cudaError_t launch_shade(const SceneView& s, const FrameView& f, const Settings&
 cudaError_t launch_connect(const SceneView& s, const FrameView& f, const Settings& st, uint32_t bounce,
                            const LaunchShape& shape, cudaStream_t stream);
 cudaError_t launch_finalize(const FrameView& f, const Settings& st, cudaStream_t stream);
-// Adds `samples` to the frame's device sample count.
-// The frame's remaining paths from `bounce` on in one launch where they are few; sets `rest` to
-// whether the launches of the remaining bounces are still to run (graph capture only).
+// The frame's remaining paths from `bounce` on in one launch: all of them, or, with `rest` (graph
+// capture), where they are few; `rest` then says whether the remaining bounces are still to run.
 cudaError_t launch_tail(const SceneView& s, const FrameView& f, const Settings& st, uint32_t bounce,
-                        const LaunchShape& shape, cudaGraphConditionalHandle rest, cudaStream_t stream);
+                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, cudaStream_t stream);
+// Adds `samples` to the frame's device sample count.
 cudaError_t launch_advance(const FrameView& f, uint32_t samples, cudaStream_t stream);
 // One bounce of a debug render mode (Settings::renderMode != path tracing):
 // closest hit of every ray of queue state[bounce & 1], then the mode's shade.
