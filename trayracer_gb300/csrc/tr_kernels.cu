@@ -1534,20 +1534,58 @@ __global__ void __launch_bounds__(256) finalize_kernel(FrameView f, Settings st)
 // slot (no compaction: the ambient-occlusion and wireframe modes act on
 // missed rays too). Each path sets its radiance (one contribution per path).
 
-// Closest hit of every ray of the bounce's queue (state[bounce & 1]); the
-// wireframe mode re-aims secondary rays at a jittered point of the pixel as
-// the Secondary raygen program does (optix.cu:292-300). Persistent warps with
-// lane refill as extend_kernel (a thread a ray left a warp waiting for its
-// longest ray: 720p occlusion image of a heightfield 347 -> 340 us, alone on the
-// GPU 583 -> 501 us).
+// One ray of the other render modes' queue (state[bounce & 1]); the wireframe mode re-aims secondary
+// rays at a jittered point of the pixel as the Secondary raygen program does (optix.cu:292-300).
+__device__ __forceinline__ void debug_ray(const FrameView& f, const Camera& cam, const Settings& st, uint32_t bounce,
+                                          uint32_t i, float3& O, float3& D)
+{
+    const float4* __restrict__ q = f.state[bounce & 1u];
+    const float4 O4 = q[i];
+    O = f3(O4);
+    D = f3(q[i + f.capacity]);
+    if (st.renderMode == kModeWireframe && bounce > 0) {
+        const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
+        const uint32_t pixelIx = pathIx % (f.resX * f.resY);
+        RefRng rng{tea2(st.seed + pathIx, (*f.sampleCount << 1) | 1u)};
+        float T;
+        camera_ray(cam, f.resX, f.resY, pixelIx % f.resX, pixelIx / f.resX, rng,
+                   (st.flags & TR_FLAG_REFERENCE_DRAW_RTL) != 0, O, D, T);
+    }
+}
+__device__ __forceinline__ uint4 debug_hit(const SceneView& s, uint32_t slot, uint32_t inst, float u, float v, float t)
+{
+    return slot != 0xffffffffu ? make_uint4(encode_bary(u, v), inst, __float_as_uint(__ldg(s.bvhTris + 3u * slot).w),
+                                            __float_as_uint(t))
+                               : make_uint4(0u, 0xffffffffu, 0xffffffffu, __float_as_uint(kDstMax));
+}
+
+// Closest hit of every ray of the bounce's queue, a thread a ray: for queues that leave the lane
+// refill below nothing to refill with.
+template <bool TL, int LAYOUT>
+__global__ void __launch_bounds__(128) debug_extend_once_kernel(SceneView s, FrameView f, Camera cam, Settings st,
+                                                                uint32_t bounce)
+{
+    stamp(f, kStampExtend + bounce);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= queue_length(f, bounce))
+        return;
+    float3 O, D;
+    debug_ray(f, cam, st, bounce, i, O, D);
+    float tmax = kDstMax, u = 0.f, v = 0.f;
+    uint32_t slot = 0xffffffffu, inst = 0;
+    if (!traverse_layout<false, false, TL, LAYOUT>(s, O, D, st.rayEpsilon, tmax, slot, u, v, nullptr, inst))
+        atomicOr(f.errorFlag, 1u);
+    f.hits[i] = debug_hit(s, slot, inst, u, v, tmax);
+}
+
+// The same with persistent warps and lane refill as extend_kernel (a thread a ray leaves a warp
+// waiting for its longest ray).
 template <bool TL, int LAYOUT>
 __global__ void __launch_bounds__(128, 8) debug_extend_kernel(SceneView s, FrameView f, Camera cam, Settings st,
                                                               uint32_t bounce)
 {
     stamp(f, kStampExtend + bounce);
     const uint32_t count = queue_length(f, bounce);
-    const float4* __restrict__ q = f.state[bounce & 1u];
-    const uint32_t cap = f.capacity;
     uint32_t* work = f.counters + kExtendWorkBase + bounce;
     const uint32_t lane = lane_id();
     __shared__ uint32_t rayIx[kTraversalThreadsMax];  // queue entry of this thread's ray
@@ -1563,28 +1601,16 @@ __global__ void __launch_bounds__(128, 8) debug_extend_kernel(SceneView s, Frame
         if (ended) {
             if (!base(t).ok)
                 atomicOr(f.errorFlag, 1u);
-            const uint32_t slot = base(t).hitSlot;
             f.hits[rayIx[threadIdx.x]] =
-                slot != 0xffffffffu ? make_uint4(encode_bary(base(t).u, base(t).v), hit_instance(t),
-                                                 __float_as_uint(__ldg(s.bvhTris + 3u * slot).w),
-                                                 __float_as_uint(base(t).tmax))
-                                    : make_uint4(0u, 0xffffffffu, 0xffffffffu, __float_as_uint(kDstMax));
+                debug_hit(s, base(t).hitSlot, hit_instance(t), base(t).u, base(t).v, base(t).tmax);
             ended = false;
         }
         if (idle) {
             first = __shfl_sync(kFull, first, leader);
             const uint32_t i = first + __popc(idle & ((1u << lane) - 1u));
             if (!alive && i < count) {
-                const float4 O4 = q[i];
-                float3 O = f3(O4), D = f3(q[i + cap]);
-                if (st.renderMode == kModeWireframe && bounce > 0) {
-                    const uint32_t pathIx = path_ix(__float_as_uint(O4.w));
-                    const uint32_t pixelIx = pathIx % (f.resX * f.resY);
-                    RefRng rng{tea2(st.seed + pathIx, (*f.sampleCount << 1) | 1u)};
-                    float T;
-                    camera_ray(cam, f.resX, f.resY, pixelIx % f.resX, pixelIx / f.resX, rng,
-                               (st.flags & TR_FLAG_REFERENCE_DRAW_RTL) != 0, O, D, T);
-                }
+                float3 O, D;
+                debug_ray(f, cam, st, bounce, i, O, D);
                 rayIx[threadIdx.x] = i;
                 traversal_begin<LAYOUT>(t, O, D, kDstMax);
                 alive = true;
@@ -2559,18 +2585,33 @@ cudaError_t launch_adjoint(const SceneView& s0, const FrameView& f, const Camera
     return e != cudaSuccess ? e : launched;
 }
 
+// Rays per SM up to which the other modes' closest hits go a thread a ray. The lane refill's larger
+// kernel, its cursor and its spills cost a small image more than the lanes it refills give
+// (320 x 180, closed room, normals 31 us, 23 a thread a ray; 1000 x 600 60 and 54 us, occlusion of
+// a heightfield 327 and 313 us); a large one of incoherent rays gains (1080p occlusion of 1.5 M
+// triangles 1259 and 1320 us, at 720p 669 and 689 us).
+constexpr uint32_t kDebugOncePerSm = 4096u;
+
 cudaError_t launch_debug_bounce(const SceneView& s0, const FrameView& f, const Camera& cam, const Settings& st,
                                 uint32_t bounce, const LaunchShape& shape, cudaStream_t stream)
 {
     const SceneView s = traced(s0, st);
     const uint32_t blocks = shape.sms * 8u;
-    const auto extend = s.tlasNodes ? (s.quantNodes ? debug_extend_kernel<true, kLayoutQuant>
-                                                    : debug_extend_kernel<true, kLayoutWide>)
-                                    : (s.quantNodes ? debug_extend_kernel<false, kLayoutQuant>
-                                                    : debug_extend_kernel<false, kLayoutWide>);
     Settings traced_st = st;
     traced_st.refillBelow = shape.refillBelow;
-    extend<<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, cam, traced_st, bounce);
+    if (f.pathCount <= shape.sms * kDebugOncePerSm) {
+        const auto extend = s.tlasNodes ? (s.quantNodes ? debug_extend_once_kernel<true, kLayoutQuant>
+                                                        : debug_extend_once_kernel<true, kLayoutWide>)
+                                        : (s.quantNodes ? debug_extend_once_kernel<false, kLayoutQuant>
+                                                        : debug_extend_once_kernel<false, kLayoutWide>);
+        extend<<<(f.pathCount + 127u) / 128u, 128, 0, stream>>>(s, f, cam, traced_st, bounce);
+    } else {
+        const auto extend = s.tlasNodes ? (s.quantNodes ? debug_extend_kernel<true, kLayoutQuant>
+                                                        : debug_extend_kernel<true, kLayoutWide>)
+                                        : (s.quantNodes ? debug_extend_kernel<false, kLayoutQuant>
+                                                        : debug_extend_kernel<false, kLayoutWide>);
+        extend<<<shape.extendBlocks, shape.traversalThreads, 0, stream>>>(s, f, cam, traced_st, bounce);
+    }
     debug_shade_kernel<<<blocks, 128, 0, stream>>>(s, f, cam, st, bounce);
     return cudaGetLastError();
 }
