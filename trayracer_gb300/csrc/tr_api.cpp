@@ -1321,7 +1321,7 @@ tr_status tr_autotune(void* ctx, void* stream, uint32_t flags, tr_tune_report* r
         if (st == TR_OK && d >= 1 && d != best.connect_blocks_per_sm)
             st = tryTuning(t);
     }
-    for (uint32_t w : {1u, 2u, 8u}) {
+    for (uint32_t w : {1u, 2u, 4u, 8u}) {
         tr_tuning t = best;
         t.shade_waves = w;
         if (st == TR_OK && w != best.shade_waves)
