@@ -619,6 +619,8 @@ Cwbvh collapse_to_cwbvh(const BinaryBvh& bvh, const float* positions, const uint
 }
 float largest_extent(const WideNode& root)
 {
+    if ((root.hdr.z | root.hdr.w) == 0u)
+        return INFINITY;  // no child: nothing to be tested
     float most = 0.f;
     for (int a = 0; a < 3; ++a) {
         float lo = INFINITY, hi = -INFINITY;  // (empty slots are +inf .. -inf)

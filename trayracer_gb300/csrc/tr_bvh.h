@@ -73,7 +73,7 @@ bool quantize_nodes(const std::vector<WideNode>& nodes, std::vector<QuantNode>& 
 // distances are denormal below 2^-26 along the ray, with steps of 2^-49: in a scene of this
 // extent still finer than the rounding of its coordinates' differences.
 constexpr float kQuantMinExtent = 0x1p-33f;
-// The longest axis of the box of a BVH's root node.
+// The longest axis of the box of a BVH's root node (infinite without triangles).
 float largest_extent(const WideNode& root);
 // Largest magnification of a ray's direction into an instance's space that the
 // quantized layout takes (its reciprocal, at the traversal's scale, must not be
