@@ -60,6 +60,8 @@ def parse():
     p.add_argument("--profile", action="store_true",
                    help="render one eager step of the workload (spp samples as one continuous wavefront) and "
                         "exit (the case the ncu captures use)")
+    p.add_argument("--bvh-nodes", type=int, default=0, choices=[0, 1, 2],
+                   help="with --profile: node layout of the plain workload's BVH (tr_tuning.bvh_nodes)")
     p.add_argument("--workload", default="plain", choices=["plain", "batch", "adjoint", "large"],
                    help="plain: the heightfield (default); batch: the 64-scene mix in one wavefront against "
                         "per-scene renders; adjoint: forward frame and path-replay adjoint of the "
@@ -711,6 +713,8 @@ def main():
     stream = torch.cuda.current_stream()
     sptr = stream.cuda_stream
     if args.profile:
+        if args.bvh_nodes:
+            r.SetTuning(bvh_nodes=args.bvh_nodes)
         r.RenderSamples(args.spp, stream=sptr, use_graph=False)
         s = r.Statistics()
         print(json.dumps({k: s[k] for k in ("path_count", "primary_path_count", "secondary_path_count",
@@ -817,18 +821,19 @@ def main():
     achieved = ext_bytes / ext_s / 1e9
     compulsory = (ext_rays * EXTEND_BYTES_PER_RAY + hit_rays * EXTEND_BYTES_PER_HIT) / ext_s / 1e9
     # DRAM bytes per extend ray measured by ncu over all extend launches of one eager step of
-    # this workload (one pass), scaled to this run's average launch by its extend rays; labelled
-    # with its source in the line, not measured in this run
+    # this workload in the node layout in use (one pass), scaled to this run's average launch by
+    # its extend rays; labelled with its source in the line, not measured in this run
     traffic, traffic_source = None, None
+    layout = {1: "fp32", 2: "quantized"}[r.Tuning()["bvh_nodes"]]
     prof = ROOT / "profiles" / "extend_kernel_heightfield_1920x1080_traffic.txt"
     if prof.exists():
         for line in prof.read_text().splitlines():
-            if line.strip().startswith("dram_bytes_per_extend_ray:"):
+            if line.strip().startswith(f"dram_bytes_per_extend_ray_{layout}:"):
                 try:
                     traffic = float(line.split(":", 1)[1]) * ext_rays / launches
                     traffic_source = ("ncu dram__bytes_read.sum + dram__bytes_write.sum over the 15 extend "
-                                      "launches of one eager step of this workload, per extend ray, scaled to "
-                                      "this run's extend rays per launch")
+                                      f"launches of one eager step of this workload with {layout} nodes, per extend "
+                                      "ray, scaled to this run's extend rays per launch")
                 except ValueError:
                     traffic = None
 
