@@ -324,8 +324,9 @@ typedef struct tr_tuning {
     uint32_t shade_threads;         /* threads per block of the shade launches: 64 or 128 */
     uint32_t bvh_nodes;             /* node layout: 0 auto (fp32 child boxes for one-level scenes of up
                                        to 64 MB of them, else 8-bit quantized), 1 fp32 (208 B a
-                                       node), 2 quantized (80 B); tr_get_tuning reports the layout in use
-                                       (1 or 2) */
+                                       node), 2 quantized (80 B); scenes that the quantized layout's
+                                       range does not take keep fp32 ones; tr_get_tuning reports the
+                                       layout in use (1 or 2) */
 } tr_tuning;
 
 typedef struct tr_tune_report {

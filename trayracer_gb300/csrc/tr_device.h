@@ -310,7 +310,7 @@ constexpr uint32_t kTailTaken = kConnectWorkBase + TR_MAX_DEPTH;
 
 // Launches of an eager frame whose start times are kept (FrameView::stamps, nanoseconds of the
 // device's timer): a stage lasts from its launch to the next one's. Three events a bounce
-// instead held a 317 x 211 frame of 16 bounces for 665 us in place of 574.
+// instead held a 317 x 211 frame of 16 bounces for 667 us in place of 562.
 constexpr uint32_t kStampExtend = 0, kStampShade = TR_MAX_DEPTH, kStampConnect = 2 * TR_MAX_DEPTH,
                    kStampGenerate = 3 * TR_MAX_DEPTH, kStampFinalize = kStampGenerate + 1,
                    kStampEnd = kStampGenerate + 2, kStamps = kStampGenerate + 3;
