@@ -495,99 +495,116 @@ tr_status enqueue_frame(Context* c, cudaStream_t s, bool timed)
     return TR_OK;
 }
 
-// Where a captured path-traced frame hands its remaining paths to one launch (tail_kernel).
+// Where a captured path-traced frame may hand its remaining paths to one launch (tail_kernel).
 struct TailPlan {
-    uint32_t bounce = 0;       // 0: nowhere
-    bool conditional = false;  // the launches of the bounces after it stand behind a graph condition
+    uint32_t bounces[2] = {0, 0};  // 0: nowhere (more)
+    bool conditional = false;      // the launches of the bounces that follow stand behind a graph condition
+    uint32_t steadyMax = 0;        // paths taken at most where hardly any end from bounce to bounce
 };
 
 // A frame of at most kTailAlways paths hands them over for sure, and its later launches need not be
 // captured at all (60 x 60, 16 bounces 335 -> 209 us, captured anew each frame 540 -> 269 us). A
 // larger one needs a condition, which costs each capture some 20 us and each frame that keeps its
-// launches 20 us (256 x 256, 5 bounces 141 -> 163 us); it pays where the paths fade: under a sky
-// (960 x 540, 4 spp, 8 bounces 1743 -> 1414 us), or some bounces after Russian roulette sets in with
-// enough bounces to follow (300 x 300, 11 bounces, roulette from 3: 258 -> 191 us). Not in closed
-// rooms without roulette (180 x 180, 16 bounces 369 us, 437 handed over); open scenes without a sky
-// cannot be told from them here. Frames of more paths fade to few some bounces later.
+// launches 20 us and the overlap of one connect launch (256 x 256, 5 bounces 141 -> 163 us).
+// It pays where the paths fade: under a sky (960 x 540, 4 spp, 8 bounces 1743 -> 1414 us), or some
+// bounces after Russian roulette sets in (300 x 300, 11 bounces, roulette from 3: 258 -> 191 us);
+// and where each launch is as long as a slow ray, in a BVH of kDeepNodes and more (640 x 360 terrain
+// of 13 000 nodes, 16 bounces without roulette 779 -> 480 us; a closed room of 2500 nodes, 180 x 180,
+// 773 -> 680 us, but 534 -> 586 us where 50 000 paths are too many). Not in small closed rooms
+// without roulette (180 x 180, 16 bounces 369 us, 437 handed over). Frames of more paths fade to few
+// some bounces later; scenes of many nodes get a second chance there, since terrain fades at once
+// and a room with roulette does not.
 constexpr uint32_t kTailAlways = 4096;
-TailPlan tail_plan(const Settings& st, uint32_t paths, bool sky)
+constexpr uint32_t kDeepNodes = 64;
+TailPlan tail_plan(const Settings& st, uint32_t paths, const SceneView& scene, uint32_t nodes)
 {
+    const bool deep = nodes >= kDeepNodes;
+    const bool roulette = st.rrStart < TR_MAX_DEPTH;
     TailPlan plan;
-    uint32_t follow = 0;  // bounces that have to follow
-    if (paths <= kTailAlways) {
-        plan.bounce = 3;
+    plan.conditional = paths > kTailAlways;
+    plan.steadyMax = deep ? kTailPaths : kTailPathsSteady;
+    uint32_t follow = deep ? 2 : 4;  // bounces that have to follow
+    if (!plan.conditional) {
+        plan.bounces[0] = 3;
         follow = 3;
-    } else if (sky) {
-        plan.bounce = paths <= (1u << 22) ? 3u : 4u;
-        plan.conditional = true;
-        follow = 2;
-    } else if (st.rrStart < TR_MAX_DEPTH) {
-        plan.bounce = std::max(3u, st.rrStart + 1u) + (paths > (1u << 17) ? 2u : 0u);
-        plan.conditional = true;
-        follow = 4;
+    } else if (scene.sky.enabled) {
+        plan.bounces[0] = 3;
+        plan.bounces[1] = paths > (1u << 22) ? 6u : 0u;
+    } else if (deep) {
+        plan.bounces[0] = 3;
+        if (paths > (roulette ? 1u << 18 : 1u << 20))
+            plan.bounces[1] = 6;
+        else if (roulette && paths > kTailPaths * 3u / 2u)
+            plan.bounces[1] = std::max(4u, st.rrStart + 1u);
+    } else if (roulette) {
+        plan.bounces[0] = std::max(3u, st.rrStart + 1u) + (paths > (1u << 17) ? 2u : 0u);
     }
     const bool counting = (st.flags & TR_FLAG_COUNT_TRAVERSAL) != 0;  // (tail_kernel keeps no such counts)
-    return plan.bounce && !counting && st.maxDepth >= plan.bounce + follow ? plan : TailPlan{};
+    for (uint32_t& b : plan.bounces)
+        if (counting || b + follow > st.maxDepth)
+            b = 0;
+    return plan;
 }
 
-// A path-traced frame with a tail_kernel launch as a graph.
+// A path-traced frame with tail_kernel launches as a graph.
 tr_status capture_frame(Context* c, cudaGraph_t g, const TailPlan& plan)
 {
     cudaStream_t s = c->stream;
     tr_status st = TR_OK;
     auto check = [&](cudaError_t e, const char* what) { st = e == cudaSuccess ? TR_OK : cuda_fail(c, e, what); };
     cudaGraphNode_t last = nullptr;
-    // captures body() after the last node; one kernel ends each: the next one's only dependency
-    auto capture = [&](auto&& body) -> tr_status {
+    // captures body() into `into` after `*after`; one kernel ends each: the next one's only dependency
+    auto capture = [&](cudaGraph_t into, cudaGraphNode_t* after, auto&& body) -> tr_status {
         const cudaError_t e = capture_into(
-            s, g, last ? &last : nullptr, last ? 1 : 0,
+            s, into, after && *after ? after : nullptr, after && *after ? 1 : 0,
             [&]() {
                 body();
                 return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
             },
-            &last);
+            after);
         if (st != TR_OK)
             return st;
         TR_CUDA(c, e);
         return TR_OK;
     };
-    auto finalize = [&]() { check(launch_finalize(c->frame, c->settings, s), "launch_finalize"); };
-    cudaGraphConditionalHandle rest{};  // whether the bounces after the tail launch are still to run
-    if (plan.conditional)
-        TR_CUDA(c, cudaGraphConditionalHandleCreate(&rest, g, 0u, cudaGraphCondAssignDefault));
-    tr_status cs = capture([&]() {
-        st = enqueue_begin(c, s);
-        if (st == TR_OK && (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING))
-            check(launch_generate(c->frame, c->camera, c->settings, s), "launch_generate");
-        if (st == TR_OK)
-            st = enqueue_bounces(c, s, 0, plan.bounce, false);
-        if (st == TR_OK)
-            check(launch_tail(c->scene, c->frame, c->settings, plan.bounce, c->shape,
-                              plan.conditional ? &rest : nullptr, s), "launch_tail");
-        if (st == TR_OK && !plan.conditional)
-            finalize();
-    });
-    if (cs != TR_OK || !plan.conditional)
-        return cs;
-    cudaGraphNodeParams cp{};
-    cp.type = cudaGraphNodeTypeConditional;
-    cp.conditional.handle = rest;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node = nullptr;
-    TR_CUDA(c, cudaGraphAddNode(&node, g, &last, nullptr, 1, &cp));
-    last = node;
-    const cudaError_t e = capture_into(
-        s, cp.conditional.phGraph_out[0], nullptr, 0,
-        [&]() {
-            st = enqueue_bounces(c, s, plan.bounce, c->settings.maxDepth, false);
-            return st == TR_OK ? cudaSuccess : cudaErrorUnknown;
-        },
-        nullptr);
-    if (st != TR_OK)
-        return st;
-    TR_CUDA(c, e);
-    return capture(finalize);
+    cudaGraphConditionalHandle rest{};  // whether the bounces after the last tail launch are still to run
+    for (uint32_t from = 0, k = 0, to = 0;; from = to, ++k) {
+        const uint32_t tail = k < 2u ? plan.bounces[k] : 0u;
+        to = tail ? tail : c->settings.maxDepth;
+        // the bounces [from, to): behind the condition of the tail launch before them
+        if (from > 0) {
+            cudaGraphNodeParams cp{};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = rest;
+            cp.conditional.type = cudaGraphCondTypeIf;
+            cp.conditional.size = 1;
+            cudaGraphNode_t node = nullptr;
+            TR_CUDA(c, cudaGraphAddNode(&node, g, &last, nullptr, 1, &cp));
+            last = node;
+            const tr_status cs = capture(cp.conditional.phGraph_out[0], nullptr,
+                                         [&]() { st = enqueue_bounces(c, s, from, to, false); });
+            if (cs != TR_OK)
+                return cs;
+        }
+        if (tail && plan.conditional)
+            TR_CUDA(c, cudaGraphConditionalHandleCreate(&rest, g, 0u, cudaGraphCondAssignDefault));
+        const tr_status cs = capture(g, &last, [&]() {
+            if (from == 0) {
+                st = enqueue_begin(c, s);
+                if (st == TR_OK && (c->settings.flags & TR_FLAG_REFERENCE_SAMPLING))
+                    check(launch_generate(c->frame, c->camera, c->settings, s), "launch_generate");
+                if (st == TR_OK)
+                    st = enqueue_bounces(c, s, 0, to, false);
+            }
+            if (st == TR_OK && tail)
+                check(launch_tail(c->scene, c->frame, c->settings, tail, c->shape,
+                                  plan.conditional ? &rest : nullptr, plan.steadyMax, s), "launch_tail");
+            if (st == TR_OK && (!tail || !plan.conditional))
+                check(launch_finalize(c->frame, c->settings, s), "launch_finalize");
+        });
+        if (cs != TR_OK || !tail || !plan.conditional)
+            return cs;
+    }
 }
 
 } // namespace
@@ -1552,9 +1569,9 @@ tr_status tr_render_frame(void* ctx, void* stream, int32_t use_graph)
             cudaGraph_t g = nullptr;
             cudaError_t ec;
             const TailPlan plan = c->renderMode == kModePathTracing
-                                      ? tail_plan(c->settings, c->frame.pathCount, c->scene.sky.enabled)
+                                      ? tail_plan(c->settings, c->frame.pathCount, c->scene, c->info.bvh_node_count)
                                       : TailPlan{};
-            if (plan.bounce) {
+            if (plan.bounces[0]) {
                 TR_CUDA(c, cudaGraphCreate(&g, 0));
                 st = capture_frame(c, g, plan);
                 ec = cudaSuccess;

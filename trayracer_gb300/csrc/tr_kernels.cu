@@ -1400,12 +1400,11 @@ __global__ void __launch_bounds__(128, TL ? 7 : 9) connect_kernel(SceneView s, F
 // the same order), without queues; or, if there are too many, it only sets the condition under
 // which the frame's graph goes on with them. A warp takes as few paths as fill the grid: their
 // divergent loops then hardly wait for one another.
-// Too many are more than kTailPaths, and more than kTailPathsSteady where more than two thirds of
-// the last bounce's paths are still there: those go on for many bounces, and a lane whose path ends
-// stays empty (closed room without roulette, 16 bounces: 2500 paths at bounce 3 375 -> 223 us, 6900
-// paths 373 -> 358 us, 22 000 paths 376 -> 440 us; with roulette 20 000 paths 374 -> 290 us).
-constexpr uint32_t kTailPaths = 32768;
-constexpr uint32_t kTailPathsSteady = 4096;
+// Too many are more than kTailPaths, or more than steadyMax (kTailPathsSteady, kTailPaths in scenes
+// of many nodes) where more than two thirds of the last bounce's paths are still there: those go on
+// for many bounces, and a lane whose path ends stays empty (closed room without roulette, 16
+// bounces: 2500 paths at bounce 3 375 -> 223 us, 6900 paths 373 -> 358 us, 22 000 paths 376 -> 440
+// us; around 2500 nodes 21 000 paths 773 -> 680 us; with roulette 20 000 paths 374 -> 290 us).
 
 __device__ __noinline__ bool tail_closest(const SceneView& s, float3 O, float3 D, float tmin, float& tmax,
                                           uint32_t& slot, float& u, float& v, uint32_t& inst)
@@ -1425,13 +1424,15 @@ template <bool REF, bool TEX>
 __global__ void __launch_bounds__(128) tail_kernel(const __grid_constant__ SceneView s,
                                                    const __grid_constant__ FrameView f,
                                                    const __grid_constant__ Settings st, uint32_t bounce,
-                                                   cudaGraphConditionalHandle rest, bool conditional)
+                                                   cudaGraphConditionalHandle rest, bool conditional, uint32_t steadyMax)
 {
     using Rng = std::conditional_t<REF, RefRng, CounterRng>;
-    const uint32_t count = __ldcg(f.counters + bounce);
+    // (set to its bounce by the launch that takes the paths: blocks of it that start late see theirs)
+    const uint32_t taken = __ldcg(f.counters + kTailTaken);
+    const uint32_t count = taken != 0u && taken != bounce ? 0u : __ldcg(f.counters + bounce);
     if (conditional) {
         const bool steady = 3u * count > 2u * __ldcg(f.counters + bounce - 1u);
-        const bool many = count > (steady ? kTailPathsSteady : kTailPaths);
+        const bool many = count > (steady ? steadyMax : kTailPaths);
         if (blockIdx.x == 0 && threadIdx.x == 0)
             cudaGraphSetConditional(rest, many ? 1u : 0u);
         if (many)
@@ -2481,7 +2482,8 @@ cudaError_t launch_connect(const SceneView& s0, const FrameView& f, const Settin
 }
 
 cudaError_t launch_tail(const SceneView& s0, const FrameView& f, const Settings& st, uint32_t bounce,
-                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, cudaStream_t stream)
+                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, uint32_t steadyMax,
+                        cudaStream_t stream)
 {
     const SceneView s = traced(s0, st);
     const bool ref = (st.flags & TR_FLAG_REFERENCE_SAMPLING) != 0;
@@ -2489,7 +2491,7 @@ cudaError_t launch_tail(const SceneView& s0, const FrameView& f, const Settings&
                                    : (ref ? tail_kernel<true, false> : tail_kernel<false, false>);
     // a warp for every path up to four blocks per SM
     const uint32_t blocks = std::max((std::min(f.pathCount, kTailPaths) + 127u) / 128u, shape.sms * 4u);
-    kernel<<<blocks, 128, 0, stream>>>(s, f, st, bounce, rest ? *rest : cudaGraphConditionalHandle{}, rest != nullptr);
+    kernel<<<blocks, 128, 0, stream>>>(s, f, st, bounce, rest ? *rest : cudaGraphConditionalHandle{}, rest != nullptr, steadyMax);
     return cudaGetLastError();
 }
 

@@ -41,8 +41,12 @@ cudaError_t launch_connect(const SceneView& s, const FrameView& f, const Setting
 cudaError_t launch_finalize(const FrameView& f, const Settings& st, cudaStream_t stream);
 // The frame's remaining paths from `bounce` on in one launch: all of them, or, with `rest` (graph
 // capture), where they are few; `rest` then says whether the remaining bounces are still to run.
+// Few are kTailPaths, or `steadyMax` where more than two thirds of the last bounce's paths are left.
+constexpr uint32_t kTailPaths = 32768;
+constexpr uint32_t kTailPathsSteady = 4096;
 cudaError_t launch_tail(const SceneView& s, const FrameView& f, const Settings& st, uint32_t bounce,
-                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, cudaStream_t stream);
+                        const LaunchShape& shape, const cudaGraphConditionalHandle* rest, uint32_t steadyMax,
+                        cudaStream_t stream);
 // Adds `samples` to the frame's device sample count.
 cudaError_t launch_advance(const FrameView& f, uint32_t samples, cudaStream_t stream);
 // One bounce of a debug render mode (Settings::renderMode != path tracing):
